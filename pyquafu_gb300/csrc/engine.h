@@ -108,7 +108,8 @@ struct KOp {
     uint32_t coef;  // offset into the coefficient pool (in reals)
     uint8_t tk[MAXK];
     uint8_t pad2[2];
-    uint32_t xreg;  // K_PROBE: flip mask over register bits (or over global bits in whole-state passes)
+    uint32_t xreg;  // K_PROBE: flip mask over register bits (or over global bits in whole-state passes);
+                    // K_DIAGR: the register bits its entries depend on
 };
 static_assert(sizeof(KOp) == 48, "KOp layout");
 

@@ -247,7 +247,7 @@ void jit_set_config(const JitConfig& c) {
 
 // The shape a plan's passes are compiled with: the configured or automatic
 // register budget (shape_for), coefficients in the kernel parameters when no
-// bind rewrites the pool on the device, the bounds mode, the float-pair
+// bind rewrites the pool on the device (not for FP64), the bounds mode, the float-pair
 // chain, and double buffering only where the register budget's resident
 // CTAs (minb) still fit in the SM's shared memory with two tiles each
 // (otherwise the second buffer costs a resident CTA: measured 1.5x slower
@@ -256,7 +256,10 @@ void jit_set_config(const JitConfig& c) {
 JitShape plan_shape(const qfvm_plan* p, int nstates, size_t optin, size_t per_sm) {
     const HostPlan& hp = p->hp;
     JitShape sh = shape_for(hp, nstates);
-    sh.pcoef = hp.binds.empty() ? 1 : 0;
+    // FP64 passes read the pool: they are bound by the FP64 pipe, and its FMAs
+    // ran slower with constant operands (25 qubits, 30 layers: 60.1 ms with
+    // the parameter block, 55.3 ms without)
+    sh.pcoef = hp.binds.empty() && hp.arith != QFVM_C128 ? 1 : 0;
     sh.bounds = bounds_check_env();
     sh.chain = p->chain_ok ? chain_for(hp, sh) : 0;
     JitShape two_sh = sh;
@@ -413,22 +416,24 @@ int prepare_impl(qfvm_plan* p, int nstates, std::string* err) {
     // the coefficient parameter blocks of the compiled passes
     p->jit_cblob[si].assign(hp.passes.size(), {});
     for (size_t i = 0; i < hp.passes.size(); ++i) {
-        uint32_t lo = 0, hi = 0;
-        if (!ks[i] || !jit_pass_coef_block(hp, static_cast<int>(i), sh, &lo, &hi)) continue;
+        std::vector<uint32_t> entries;
+        if (!ks[i] || !jit_pass_coef_block(hp, static_cast<int>(i), sh, &entries)) continue;
         std::vector<unsigned char>& blob = p->jit_cblob[si][i];
-        const size_t eb = hp.arith == QFVM_C64 ? 4 : 8;
-        blob.assign(((hi - lo) * eb + 15) / 16 * 16, 0);
-        for (uint32_t c = lo; c < hi; ++c) {
-            const double v = hp.coef[c];
-            unsigned char* d = blob.data() + (c - lo) * eb;
+        // floats twice in a row: the kernels read packed pairs of them
+        const size_t eb = hp.arith == QFVM_C128_DS ? 16 : 8;
+        blob.assign((entries.size() * eb + 15) / 16 * 16, 0);
+        for (size_t e = 0; e < entries.size(); ++e) {
+            const double v = hp.coef[entries[e]];
+            unsigned char* d = blob.data() + e * eb;
             if (hp.arith == QFVM_C64) {
                 const float f = static_cast<float>(v);
                 std::memcpy(d, &f, 4);
+                std::memcpy(d + 4, &f, 4);
             } else if (hp.arith == QFVM_C128_DS) {
                 const float h = static_cast<float>(v);
                 const float l = static_cast<float>(v - static_cast<double>(h));
-                std::memcpy(d, &h, 4);
-                std::memcpy(d + 4, &l, 4);
+                const float quad[4] = {h, h, l, l};
+                std::memcpy(d, quad, 16);
             } else {
                 std::memcpy(d, &v, 8);
             }
@@ -530,13 +535,14 @@ cudaError_t jit_launch_pass(qfvm_plan* p, int pi, void* psi, void* lam, const vo
     void* a_part = partial;
     uint64_t a_wait = g_wait_ns.load();
     uint32_t a_extra = g_extra_tx.load();
+    uint64_t a_zero2 = 0;
     // the coefficient block (when the kernel takes one) is its last parameter
     const std::vector<std::vector<unsigned char>>& blobs = p->jit_cblob[si];
     void* a_blob = (pi < static_cast<int>(blobs.size()) && !blobs[pi].empty())
                        ? const_cast<unsigned char*>(blobs[pi].data())
                        : nullptr;
     void* args[] = {&a_psi, &a_lam, &ntiles, &a_coef, &a_cs, &a_ish, &a_act, &a_pt, &a_part, &a_status, &a_wait, &a_extra,
-                    a_blob};
+                    &a_zero2, a_blob};
     CUresult r = driver().launch(k->fn, grid, 1, 1, k->threads, 1, 1, static_cast<unsigned>(k->smem),
                                  reinterpret_cast<CUstream>(st), args, nullptr);
     if (grid_out) *grid_out = static_cast<int>(grid);

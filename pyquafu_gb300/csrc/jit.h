@@ -9,6 +9,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <vector>
 
 #include "engine.h"
 
@@ -41,10 +42,10 @@ bool jit_pass_ptx(const HostPlan& hp, int pi, const JitShape& sh, const std::str
                   std::string* why);
 
 // Parameter-block coefficients of pass `pi` (sh.pcoef): true with the pool
-// range [cmin, cmax) the kernel takes as its last parameter p_cblob (in the
-// arithmetic's format: float, float pair or double per pool entry); false
+// entries, in order, that the kernel takes as its last parameter p_cblob (in
+// the arithmetic's format: a double, or every float twice in a row); false
 // when the pass reads them from the pool in global memory.
-bool jit_pass_coef_block(const HostPlan& hp, int pi, const JitShape& sh, uint32_t* cmin, uint32_t* cmax);
+bool jit_pass_coef_block(const HostPlan& hp, int pi, const JitShape& sh, std::vector<uint32_t>* entries);
 
 // Dynamic shared memory of a specialised pass: nb tile slots of nstates
 // tiles in the padded tile layout, the per-warp probe sums, one mbarrier per

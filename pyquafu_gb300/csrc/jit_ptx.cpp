@@ -1,15 +1,29 @@
 // PTX generator of circuit-specialised tile passes (see jit.h).
 //
 // The emitted kernel is the tile pass of device.cuh (k_pass) / adjoint.cuh
-// (k_pass2) with the plan's steps unrolled: the persistent tile loop, the
-// cp.async staging of a tile into swizzled shared memory, for every
-// register round the loads, the gate arithmetic and the stores, all with
-// compile-time register indices, and two-target dense gates as
-// shared-memory steps over the tile.  The gate arithmetic follows the policy
-// primitives of policy.cuh operation for operation (mul.rn / fma.rn / add.rn,
-// no contraction), so the specialised passes compute what the interpreting
-// kernels compute.  Register permutations (X, SWAP, Y, quarter turns) are
-// renames of PTX virtual registers and cost no instruction.
+// (k_pass2) with the plan's steps unrolled: the persistent tile loop, bulk
+// copies of a tile into padded shared memory, for every register round the
+// loads, the gate arithmetic and the stores, all with compile-time register
+// indices, and two-target dense gates as shared-memory steps.  Register
+// permutations (X, SWAP, Y, quarter turns) are renames of PTX virtual
+// registers and cost no instruction.
+//
+// FP64 gate arithmetic follows the primitives of policy.cuh operation for
+// operation (mul.rn / fma.rn / add.rn, no contraction); so does complex64,
+// with both floats of an amplitude in one packed instruction where they meet
+// the same coefficient.  Double-single arithmetic is packed throughout.
+//
+// What bounds the passes (152 SMs, 1.92 GHz; microbenchmarks of the packed
+// and scalar FP32 instructions): an SM sub-partition issues one instruction
+// and reads two 32-bit register operands per lane and clock, whatever pipe
+// they go to.  A packed instruction with two register operands takes 2
+// clocks (0.98 of that measured), with three 3; one whose third operand is a
+// constant stays at 2.  So packing halves the issue slots, coefficients
+// belong into the parameter block, and the remaining cost is the register
+// operands of the arithmetic itself.  Measured on the benchmark family,
+// scalar arithmetic and coefficients mostly loaded per thread before:
+// 30 qubits float pairs 1057 -> 939 ms, 27 qubits complex64 20.4 -> 18.2 ms,
+// 24-qubit float-pair gradient 133 -> 101 ms.
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -32,10 +46,30 @@ std::string fmt(const char* f, ...) {
     return buf;
 }
 
+// A complex amplitude: its real registers x, y, and (complex64, double-single)
+// its packed form p, one 64-bit register (re, im).  Either form may be empty
+// until it is asked for (Gen::xy, Gen::pk).  Double-single registers are
+// written "high|low".
 struct Cx {
-    std::string x, y;
+    std::string x, y, p;
+    Cx() = default;
+    Cx(std::string re, std::string im) : x(std::move(re)), y(std::move(im)) {}
+    static Cx packed(std::string v) {
+        Cx c;
+        c.p = std::move(v);
+        return c;
+    }
 };
-bool same(const Cx& a, const Cx& b) { return a.x == b.x && a.y == b.y; }
+bool same(const Cx& a, const Cx& b) {
+    if (!a.p.empty() && !b.p.empty()) return a.p == b.p;
+    return !a.x.empty() && a.x == b.x && a.y == b.y;
+}
+// coef * amp (rot 0), coef * i * amp (rot 1) or coef * -i * amp (rot 3)
+struct Term {
+    std::string c;
+    Cx* a;
+    int rot;
+};
 
 class Gen {
    public:
@@ -46,6 +80,7 @@ class Gen {
         ft_ = f64_ ? "f64" : "f32";
         es_ = (f64_ || ds_) ? 16 : 8;
         cb_ = (f64_ || ds_) ? 8 : 4;
+        pb_ = ds_ ? 16 : 8;  // a parameter-block coefficient: FP64, or every float twice (packed operands)
         T_ = hp.T;
         R_ = hp.R;
         NT_ = 1 << (T_ - R_);
@@ -66,14 +101,15 @@ class Gen {
         in_pair_ = ds_ && sh.chain && pi > 0;
         out_pair_ = ds_ && sh.chain && pi + 1 < static_cast<int>(hp.passes.size());
         bulk_out_ = !ds_ || out_pair_;
-        if (sh.pcoef) coef_range(&cmin_, &cmax_);
-        pc_ = sh.pcoef && cmax_ > cmin_ && blob_bytes() <= kMaxBlob;
+        if (sh.pcoef) coef_list();
+        pc_ = sh.pcoef && !clist_.empty() && blob_bytes() <= kMaxBlob;
     }
 
-    // Coefficient pool entries the pass's operations read: [lo, hi).
-    void coef_range(uint32_t* lo, uint32_t* hi) const {
-        *lo = ~0u;
-        *hi = 0;
+    // Coefficient pool entries the pass's operations read, in the order of
+    // the operations: entry i of the list is coefficient i of the parameter
+    // block (a plan's pool holds its merged tables apart from the gates, so
+    // the pool range of a pass can be many times what it reads).
+    void coef_list() {
         for (int si = 0; si < pd_.step_count; ++si) {
             const StepDesc& sd = hp_.steps[pd_.step_begin + si];
             for (int oi = 0; oi < sd.op_count; ++oi) {
@@ -88,21 +124,20 @@ class Gen {
                     case K_PROBE: n = 1; break;
                     default: break;
                 }
-                if (n == 0) continue;
-                if (o.coef < *lo) *lo = o.coef;
-                if (o.coef + n > *hi) *hi = o.coef + n;
+                for (int i = 0; i < n; ++i) {
+                    if (o.kind == K_DIAGR && diagr_code(o, i / 2) != DIAGR_GENERAL) continue;
+                    const uint32_t at = o.coef + static_cast<uint32_t>(i);
+                    if (cindex_.emplace(at, static_cast<uint32_t>(clist_.size())).second) clist_.push_back(at);
+                }
             }
         }
-        if (*hi == 0) *lo = 0;
     }
-    uint32_t blob_bytes() const { return ((cmax_ - cmin_) * cb_ + 15u) / 16u * 16u; }
+    uint32_t blob_bytes() const { return (static_cast<uint32_t>(clist_.size()) * pb_ + 15u) / 16u * 16u; }
+    const std::vector<uint32_t>& coef_entries() const { return clist_; }
 
     bool param_coefs() const { return pc_; }
     bool in_pairs() const { return in_pair_; }
     bool out_pairs() const { return out_pair_; }
-    uint32_t cmin() const { return cmin_; }
-    uint32_t cmax() const { return cmax_; }
-
 
     bool supported(std::string* why) const {
         if (hp_.arith != QFVM_C64 && hp_.arith != QFVM_C128 && hp_.arith != QFVM_C128_DS)
@@ -145,13 +180,14 @@ class Gen {
         out += "\t.param .u64 p_psi,\n\t.param .u64 p_lam,\n\t.param .u64 p_ntiles,\n\t.param .u64 p_coef,\n";
         out += "\t.param .u64 p_cstride,\n\t.param .u32 p_ishift,\n\t.param .u64 p_active,\n";
         out += "\t.param .u32 p_per_tile,\n\t.param .u64 p_partial,\n\t.param .u64 p_status,\n";
-        out += "\t.param .u64 p_wait_ns,\n\t.param .u32 p_extra_tx";
+        out += "\t.param .u64 p_wait_ns,\n\t.param .u32 p_extra_tx,\n\t.param .u64 p_zero2";
         if (pc_) out += fmt(",\n\t.param .align 16 .b8 p_cblob[%u]", blob_bytes());
         out += "\n)\n";
         out += fmt(".maxntid %d, 1, 1\n.minnctapersm %d\n{\n", NT_, sh_.minb < 1 ? 1 : sh_.minb);
         out += fmt("\t.reg .pred %%p<%d>;\n\t.reg .b16 %%h<%d>;\n\t.reg .b32 %%r<%d>;\n\t.reg .b64 %%rd<%d>;\n",
                    np_reg_ + 1, nh_ + 1, nr_ + 1, nrd_ + 1);
-        out += fmt("\t.reg .%s %%a<%d>;\n\t.reg .f64 %%d<%d>;\n\n", ft_, na_ + 1, nd_ + 1);
+        out += fmt("\t.reg .%s %%a<%d>;\n\t.reg .f64 %%d<%d>;\n\t.reg .b64 %%q<%d>;\n\n", ft_, na_ + 1, nd_ + 1,
+                   nq_ + 1);
         out += body_;
         out += "}\n";
         return out;
@@ -170,6 +206,7 @@ class Gen {
     std::string P() { return "%p" + std::to_string(np_reg_++); }
     std::string A() { return "%a" + std::to_string(na_++); }
     std::string D() { return "%d" + std::to_string(nd_++); }
+    std::string Q() { return "%q" + std::to_string(nq_++); }
     std::string L() { return "$L" + std::to_string(nl_++); }
     void I(const std::string& s) { Iraw(bc_ ? checked(s) : s); }
     // a comment line in the emitted PTX (marks what the following
@@ -338,26 +375,282 @@ class Gen {
         I(fmt("fma.rn.%s %s, %s, %s, %s", ft_, d.c_str(), c.c_str(), x.c_str(), acc.c_str()));
         return d;
     }
-    // sum of c_i * x_i.  FP64 / FP32: mul then fma in order (the same
-    // roundings as the nested mul / fma form).  Double-single: every product
-    // split exactly (FMA TwoProd), the products' high parts summed with
-    // TwoSum, all error terms summed in FP32, one renormalisation at the end.
-    std::string dot(const std::vector<std::pair<std::string, std::string>>& t) {
+    // ---- packed arithmetic (complex64, double-single) ----
+    // The two floats of a packed register go through one add / sub / mul /
+    // fma .f32x2 instruction: the FP32 pipe does the same work per clock, but
+    // in half the issue slots, and the passes are bound by instruction issue.
+    std::string q2(const char* op, const std::string& a, const std::string& b) {
+        std::string d = Q();
+        I(fmt("%s.rn.f32x2 %s, %s, %s", op, d.c_str(), a.c_str(), b.c_str()));
+        return d;
+    }
+    std::string q2fma(const std::string& a, const std::string& b, const std::string& c) {
+        std::string d = Q();
+        I(fmt("fma.rn.f32x2 %s, %s, %s, %s", d.c_str(), a.c_str(), b.c_str(), c.c_str()));
+        return d;
+    }
+    // A packed product that feeds a packed sum as a rounded value (float-pair
+    // arithmetic).  The assembler contracts mul.rn.f32x2 with a following
+    // add / sub .f32x2, also with the .rn on both, and also when the product
+    // is an fma with a constant zero: the addend is a zero it does not know
+    // (the kernel parameter p_zero2).
+    std::string q2mul(const std::string& a, const std::string& b) { return q2fma(a, b, zero2_); }
+    std::string join(const std::string& lo, const std::string& hi) {
+        std::string d = Q();
+        I(fmt("mov.b64 %s, {%s, %s}", d.c_str(), lo.c_str(), hi.c_str()));
+        return d;
+    }
+    std::pair<std::string, std::string> split(const std::string& q) {
+        std::string lo = A(), hi = A();
+        I(fmt("mov.b64 {%s, %s}, %s", lo.c_str(), hi.c_str(), q.c_str()));
+        return {lo, hi};
+    }
+    // the real registers of an amplitude
+    void xy(Cx& c) {
+        if (!c.x.empty()) return;
+        if (ds_) {
+            auto [H, L] = hl(c.p);
+            auto [xh, yh] = split(H);
+            auto [xl, yl] = split(L);
+            c.x = xh + "|" + xl;
+            c.y = yh + "|" + yl;
+        } else {
+            auto [re, im] = split(c.p);
+            c.x = re;
+            c.y = im;
+        }
+    }
+    // its packed register (double-single: "high pair|low pair")
+    const std::string& pk(Cx& c) {
+        if (!c.p.empty()) return c.p;
+        if (ds_) {
+            auto [xh, xl] = hl(c.x);
+            auto [yh, yl] = hl(c.y);
+            const std::string H = join(xh, yh);
+            c.p = H + "|" + join(xl, yl);
+        } else {
+            c.p = join(c.x, c.y);
+        }
+        return c.p;
+    }
+    // coefficient in both halves of a packed register: a parameter-block
+    // coefficient is stored that way, others are duplicated once
+    std::string both(const std::string& c) {
+        auto it = both_.find(c);
+        if (it != both_.end()) return it->second;
+        auto one = [&](const std::string& r, const std::string& addr) {
+            std::string d = Q();
+            if (addr.empty()) I(fmt("mov.b64 %s, {%s, %s}", d.c_str(), r.c_str(), r.c_str()));
+            else I(fmt("ld.param.b64 %s, [%s]", d.c_str(), addr.c_str()));
+            return d;
+        };
+        auto pa = param_at_.find(c);
+        const bool in_param = pa != param_at_.end();
+        std::string v;
+        if (ds_) {
+            auto [h, l] = hl(c);
+            v = one(h, in_param ? fmt("p_cblob+%u", pa->second) : "");
+            v += "|" + one(l, in_param ? fmt("p_cblob+%u", pa->second + 8) : "");
+        } else {
+            v = one(c, in_param ? fmt("p_cblob+%u", pa->second) : "");
+        }
+        both_[c] = v;
+        return v;
+    }
+    std::string negc(const std::string& c) {  // -coefficient, once per coefficient
+        auto it = negc_.find(c);
+        if (it != negc_.end()) return it->second;
+        return negc_[c] = neg(c);
+    }
+    // i^rot * amp, once per packed amplitude
+    Cx& turned(Cx& a, int rot) {
+        if (rot == 0) return a;
+        const std::string key = pk(a) + (rot == 1 ? "+" : "-");
+        auto it = turned_.find(key);
+        if (it != turned_.end()) return it->second;
+        xy(a);
+        Cx t = rot == 1 ? Cx{neg(a.y), a.x} : Cx{a.y, neg(a.x)};
+        return turned_[key] = t;
+    }
+    // Double-single c * x (+ the running pair (s, e)), packed.  With s' =
+    // fl(s + p), p = fl(ch * xh), TwoSum leaves the rounding error
+    // (s - (s' - v)) + (p - v), v = s' - s; replacing p by the exact ch * xh
+    // in one FMA adds the product's own error without forming it.
+    void ds_axpy(const std::string& c, const std::string& x, std::string* s, std::string* e) {
+        auto [ch, cl] = hl(c);
+        auto [xh, xl] = hl(x);
+        const std::string p = q2mul(ch, xh);
+        const std::string t = q2("add", *s, p);
+        const std::string nv = q2("sub", *s, t);
+        const std::string d1 = q2("sub", *s, q2("add", t, nv));
+        const std::string d2 = q2fma(ch, xh, nv);
+        std::string lo = q2fma(ch, xl, *e);
+        lo = q2fma(cl, xh, lo);
+        *e = q2("add", q2("add", d1, d2), lo);
+        *s = t;
+    }
+    // Linear combination of amplitudes with real coefficients, plus init when
+    // given.  FP64 / FP32: mul (or init) then fma in the order of the terms,
+    // the roundings of policy.cuh.  Complex64 does unturned terms packed and
+    // the turned ones (whose halves cross) on the real registers.
+    // Double-single: as ds_axpy, term by term, all packed.
+    Cx lin(std::vector<Term> t, Cx* init = nullptr) {
+        if (f64_) {
+            std::string re, im;
+            if (init) {
+                re = init->x;
+                im = init->y;
+            }
+            for (Term& k : t) {
+                const Cx& a = *k.a;
+                const std::string& u = k.rot == 0 ? a.x : a.y;
+                const std::string& v = k.rot == 0 ? a.y : a.x;
+                const std::string cu = k.rot == 1 ? negc(k.c) : k.c, cv = k.rot == 3 ? negc(k.c) : k.c;
+                re = re.empty() ? mul(cu, u) : fma(cu, u, re);
+                im = im.empty() ? mul(cv, v) : fma(cv, v, im);
+            }
+            return {re, im};
+        }
         if (!ds_) {
-            std::string acc = mul(t[0].first, t[0].second);
-            for (size_t i = 1; i < t.size(); ++i) acc = fma(t[i].first, t[i].second, acc);
+            Cx acc;
+            size_t i = 0;
+            if (init) {
+                acc = *init;
+            } else {
+                // a crossing term follows: on the real registers from the start
+                // (a packed product there made the five-qubit rounds spill)
+                Cx& a = *t[0].a;
+                if (t.size() > 1 && t[1].rot != 0) {
+                    xy(a);
+                    acc = Cx{f32op("mul", t[0].c, a.x), f32op("mul", t[0].c, a.y)};
+                } else {
+                    acc = Cx::packed(q2("mul", both(t[0].c), pk(a)));
+                }
+                i = 1;
+            }
+            for (; i < t.size(); ++i) {
+                if (t[i].rot == 0) {
+                    acc = Cx::packed(q2fma(both(t[i].c), pk(*t[i].a), pk(acc)));
+                } else {
+                    xy(acc);
+                    Cx& a = *t[i].a;
+                    xy(a);
+                    const std::string n = negc(t[i].c);
+                    const std::string& cu = t[i].rot == 1 ? n : t[i].c;
+                    const std::string& cv = t[i].rot == 1 ? t[i].c : n;
+                    acc = Cx{f32fma(cu, a.y, acc.x), f32fma(cv, a.x, acc.y)};
+                }
+            }
             return acc;
         }
-        auto [s, err] = hl(ds_mul_raw(t[0].first, t[0].second));
-        for (size_t i = 1; i < t.size(); ++i) {
-            auto [p, e] = hl(ds_mul_raw(t[i].first, t[i].second));
-            const std::string sn = f32op("add", s, p);
-            const std::string v = f32op("sub", sn, s);
-            const std::string r = f32op("add", f32op("sub", s, f32op("sub", sn, v)), f32op("sub", p, v));
-            err = f32op("add", f32op("add", err, e), r);
-            s = sn;
+        std::string s, e;
+        size_t i = 0;
+        if (init) {
+            auto [h, l] = hl(pk(*init));
+            s = h;
+            e = l;
+        } else {
+            auto [ch, cl] = hl(both(t[0].c));
+            auto [xh, xl] = hl(pk(turned(*t[0].a, t[0].rot)));
+            const std::string p0 = q2mul(ch, xh);
+            if (t.size() == 1) {
+                const std::string n = q2("sub", zero2_, p0);
+                e = q2fma(cl, xh, q2fma(ch, xl, q2fma(ch, xh, n)));
+                return Cx::packed(p0 + "|" + e);
+            }
+            // the first two products together: both products' errors come out
+            // of the two TwoSum residuals
+            auto [bh, bl] = hl(both(t[1].c));
+            auto [yh, yl] = hl(pk(turned(*t[1].a, t[1].rot)));
+            const std::string p1 = q2mul(bh, yh);
+            s = q2("add", p0, p1);
+            const std::string v = q2("sub", s, p0), nv = q2("sub", p0, s), nw = q2("sub", v, s);
+            const std::string d1 = q2fma(ch, xh, nw), d2 = q2fma(bh, yh, nv);
+            std::string lo = q2fma(cl, xh, q2("mul", ch, xl));
+            lo = q2fma(bl, yh, q2fma(bh, yl, lo));
+            e = q2("add", q2("add", d1, d2), lo);
+            i = 2;
         }
-        return s + "|" + err;
+        for (; i < t.size(); ++i) ds_axpy(both(t[i].c), pk(turned(*t[i].a, t[i].rot)), &s, &e);
+        return Cx::packed(s + "|" + e);
+    }
+    // a + b, a - b
+    Cx cadd(Cx& a, Cx& b) {
+        if (f64_) return {add(a.x, b.x), add(a.y, b.y)};
+        if (!ds_) return Cx::packed(q2("add", pk(a), pk(b)));
+        auto [ah, al] = hl(pk(a));
+        auto [bh, bl] = hl(pk(b));
+        const std::string s = q2("add", ah, bh), v = q2("sub", s, ah);
+        const std::string d = q2("add", q2("sub", ah, q2("sub", s, v)), q2("sub", bh, v));
+        return Cx::packed(s + "|" + q2("add", d, q2("add", al, bl)));
+    }
+    Cx csub(Cx& a, Cx& b) {
+        if (f64_) return {sub(a.x, b.x), sub(a.y, b.y)};
+        if (!ds_) return Cx::packed(q2("sub", pk(a), pk(b)));
+        auto [ah, al] = hl(pk(a));
+        auto [bh, bl] = hl(pk(b));
+        const std::string s = q2("sub", ah, bh), v = q2("sub", s, ah);
+        const std::string d = q2("sub", q2("sub", ah, q2("sub", s, v)), q2("add", bh, v));
+        return Cx::packed(s + "|" + q2("add", d, q2("sub", al, bl)));
+    }
+    // renormalised float pairs (TwoSum of high and low)
+    Cx cnorm(Cx& a) {
+        auto [h, l] = hl(pk(a));
+        const std::string s = q2("add", h, l), v = q2("sub", s, h);
+        return Cx::packed(s + "|" + q2("add", q2("sub", h, q2("sub", s, v)), q2("sub", l, v)));
+    }
+    Cx csel(Cx& a, Cx& b, const std::string& p) {  // p ? a : b
+        if (f64_ || a.p.empty() || b.p.empty()) {
+            xy(a);
+            xy(b);
+            return {sel(a.x, b.x, p), sel(a.y, b.y, p)};
+        }
+        auto one = [&](const std::string& u, const std::string& v) {
+            std::string d = Q();
+            I(fmt("selp.b64 %s, %s, %s, %s", d.c_str(), u.c_str(), v.c_str(), p.c_str()));
+            return d;
+        };
+        if (!ds_) return Cx::packed(one(a.p, b.p));
+        auto [ah, al] = hl(a.p);
+        auto [bh, bl] = hl(b.p);
+        const std::string h = one(ah, bh);
+        return Cx::packed(h + "|" + one(al, bl));
+    }
+    // p ? -a : a, by the sign bits
+    Cx cneg_if(Cx& a, const std::string& p) {
+        auto it = sign_.find(p);
+        if (it == sign_.end()) {
+            std::string m = R32(), w = R64();
+            I(fmt("selp.b32 %s, 0x80000000, 0, %s", m.c_str(), p.c_str()));
+            I(fmt("mov.b64 %s, {%s, %s}", w.c_str(), f64_ ? zero32().c_str() : m.c_str(), m.c_str()));
+            it = sign_.emplace(p, w).first;
+        }
+        auto one = [&](const std::string& v, bool packed) {
+            std::string d = packed ? Q() : A();
+            if (packed) {
+                I(fmt("xor.b64 %s, %s, %s", d.c_str(), v.c_str(), it->second.c_str()));
+            } else {
+                std::string t = R64(), u = R64();
+                I(fmt("mov.b64 %s, %s", t.c_str(), v.c_str()));
+                I(fmt("xor.b64 %s, %s, %s", u.c_str(), t.c_str(), it->second.c_str()));
+                I(fmt("mov.b64 %s, %s", d.c_str(), u.c_str()));
+            }
+            return d;
+        };
+        if (f64_) return {one(a.x, false), one(a.y, false)};
+        if (!ds_) return Cx::packed(one(pk(a), true));
+        auto [h, l] = hl(pk(a));
+        const std::string nh = one(h, true);
+        return Cx::packed(nh + "|" + one(l, true));
+    }
+    std::string zero32() {
+        std::string z = R32();
+        I(fmt("mov.u32 %s, 0", z.c_str()));
+        return z;
+    }
+    Cx cneg(Cx& a) {
+        xy(a);
+        return {neg(a.x), neg(a.y)};
     }
     std::string add(const std::string& x, const std::string& y) {
         if (ds_) return ds_add(x, y);
@@ -427,28 +720,33 @@ class Gen {
         consts_[v] = d;
         return d;
     }
-    // complex amplitude <-> shared memory (double-single: (re.h, re.l, im.h, im.l))
+    // complex amplitude <-> shared memory (double-single: the packed high
+    // pair, then the packed low pair: (re.h, im.h, re.l, im.l))
     Cx load_amp(const std::string& addr, uint32_t off) {
         if (ds_) {
-            std::string r[4] = {A(), A(), A(), A()};
-            I(fmt("ld.shared.v4.f32 {%s, %s, %s, %s}, [%s+%u]", r[0].c_str(), r[1].c_str(), r[2].c_str(),
-                  r[3].c_str(), addr.c_str(), off));
-            return {r[0] + "|" + r[1], r[2] + "|" + r[3]};
+            std::string h = Q(), l = Q();
+            I(fmt("ld.shared.v2.b64 {%s, %s}, [%s+%u]", h.c_str(), l.c_str(), addr.c_str(), off));
+            return Cx::packed(h + "|" + l);
+        }
+        if (!f64_) {
+            std::string q = Q();
+            I(fmt("ld.shared.b64 %s, [%s+%u]", q.c_str(), addr.c_str(), off));
+            return Cx::packed(q);
         }
         Cx c{A(), A()};
-        I(fmt("ld.shared.v2.%s {%s, %s}, [%s+%u]", ft_, c.x.c_str(), c.y.c_str(), addr.c_str(), off));
+        I(fmt("ld.shared.v2.f64 {%s, %s}, [%s+%u]", c.x.c_str(), c.y.c_str(), addr.c_str(), off));
         return c;
     }
-    void store_amp(const std::string& addr, uint32_t off, const Cx& c, const std::string& pred = "") {
+    void store_amp(const std::string& addr, uint32_t off, Cx& c, const std::string& pred = "") {
         const std::string g = pred.empty() ? "" : "@" + pred + " ";
         if (ds_) {
-            auto [xh, xl] = hl(c.x);
-            auto [yh, yl] = hl(c.y);
-            I(fmt("%sst.shared.v4.f32 [%s+%u], {%s, %s, %s, %s}", g.c_str(), addr.c_str(), off, xh.c_str(),
-                  xl.c_str(), yh.c_str(), yl.c_str()));
-            return;
+            auto [h, l] = hl(pk(c));
+            I(fmt("%sst.shared.v2.b64 [%s+%u], {%s, %s}", g.c_str(), addr.c_str(), off, h.c_str(), l.c_str()));
+        } else if (!f64_) {
+            I(fmt("%sst.shared.b64 [%s+%u], %s", g.c_str(), addr.c_str(), off, pk(c).c_str()));
+        } else {
+            I(fmt("%sst.shared.v2.f64 [%s+%u], {%s, %s}", g.c_str(), addr.c_str(), off, c.x.c_str(), c.y.c_str()));
         }
-        I(fmt("%sst.shared.v2.%s [%s+%u], {%s, %s}", g.c_str(), ft_, addr.c_str(), off, c.x.c_str(), c.y.c_str()));
     }
     // double-single <-> FP64 on the integer and FP32 pipes, no FP64
     // instruction (ds_from_double / ds_to_double of policy.cuh, step for step)
@@ -571,23 +869,25 @@ class Gen {
         return c;
     }
 
-    // Coefficients from the pass's parameter block p_cblob (pool entries
-    // cmin_ .. cmax_ in the arithmetic's format, warp-uniform constant
-    // memory), one scalar load each, so each can become a constant operand.
+    // Coefficients from the pass's parameter block p_cblob (the entries of
+    // coef_list, pb_ bytes each, warp-uniform constant memory), one
+    // scalar load each, so each can become a constant operand.  Floats are
+    // stored twice in a row, so that both() loads them as packed operands.
     std::vector<std::string> pcoefs(uint32_t off, int cnt) {
         std::vector<std::string> c;
         for (uint32_t i = off; i < off + static_cast<uint32_t>(cnt); ++i) {
-            const uint32_t rel = i - cmin_;
+            const uint32_t at = cindex_.at(i) * pb_;
             if (ds_) {
                 std::string h = A(), l = A();
-                I(fmt("ld.param.f32 %s, [p_cblob+%u]", h.c_str(), rel * cb_));
-                I(fmt("ld.param.f32 %s, [p_cblob+%u]", l.c_str(), rel * cb_ + 4));
+                I(fmt("ld.param.f32 %s, [p_cblob+%u]", h.c_str(), at));
+                I(fmt("ld.param.f32 %s, [p_cblob+%u]", l.c_str(), at + 8));
                 c.push_back(h + "|" + l);
             } else {
                 std::string r = A();
-                I(fmt("ld.param.%s %s, [p_cblob+%u]", ft_, r.c_str(), rel * cb_));
+                I(fmt("ld.param.%s %s, [p_cblob+%u]", ft_, r.c_str(), at));
                 c.push_back(r);
             }
+            if (!f64_) param_at_[c.back()] = at;
         }
         return c;
     }
@@ -669,6 +969,8 @@ class Gen {
         I(fmt("ld.param.u64 %s, [p_wait_ns]", waitns_.c_str()));
         extra_ = R32();
         I(fmt("ld.param.u32 %s, [p_extra_tx]", extra_.c_str()));
+        zero2_ = Q();
+        I(fmt("ld.param.b64 %s, [p_zero2]", zero2_.c_str()));
         if (bc_) {
             // bounds of the checked accesses: the dynamic shared memory, and
             // each state (ntiles tiles of 2^T amplitudes)
@@ -974,7 +1276,8 @@ class Gen {
                     std::string re = D(), im = D();
                     I(fmt("ld.shared.v2.f64 {%s, %s}, [%s+%u]", re.c_str(), im.c_str(), tbase.c_str(),
                           st * tileB_ + sk(k)));
-                    store_amp(tbase, st * tileB_ + sk(k), {ds_from(re), ds_from(im)});
+                    Cx c{ds_from(re), ds_from(im)};
+                    store_amp(tbase, st * tileB_ + sk(k), c);
                 }
             }
             I("bar.sync 0");
@@ -1007,8 +1310,9 @@ class Gen {
             // so |low| stays within half an ulp of high from pass to pass
             for (int k = 0; k < PER_; ++k)
                 for (int st = 0; st < NS_; ++st) {
-                    const Cx c = load_amp(tbase, st * tileB_ + sk(k));
-                    store_amp(tbase, st * tileB_ + sk(k), {ds_norm(c.x), ds_norm(c.y)});
+                    Cx c = load_amp(tbase, st * tileB_ + sk(k));
+                    c = cnorm(c);
+                    store_amp(tbase, st * tileB_ + sk(k), c);
                 }
         }
         if (ds_ && !out_pair_) {
@@ -1016,7 +1320,8 @@ class Gen {
                 std::string gp = thread_gptr(st, base);
                 for (int k = 0; k < PER_; ++k) {
                     const std::string dst = gaddr(gp, k);
-                    const Cx c = load_amp(tbase, st * tileB_ + sk(k));
+                    Cx c = load_amp(tbase, st * tileB_ + sk(k));
+                    xy(c);
                     const std::string re = ds_to(c.x), im = ds_to(c.y);
                     I(fmt("st.global.cs.v2.f64 [%s], {%s, %s}", dst.c_str(), re.c_str(), im.c_str()));
                 }
@@ -1124,27 +1429,76 @@ class Gen {
     }
 
     // ---------------------------------------------------------------- rounds
-    std::string ctl_pred(const KOp& o, const std::string& gthr) {
-        std::string t = R64(), p = P();
-        I(fmt("and.b64 %s, %s, %llu", t.c_str(), gthr.c_str(), static_cast<unsigned long long>(o.cthr)));
-        I(fmt("setp.eq.u64 %s, %s, %llu", p.c_str(), t.c_str(), static_cast<unsigned long long>(o.cthr)));
+    // A mask over global index bits (not register ones) splits into bits of
+    // the thread index and bits of the tile's base.
+    struct Split {
+        uint32_t thr;
+        uint64_t tile;
+    };
+    Split split_mask(uint64_t m) const {
+        Split r{0, m};
+        for (int k = 0; k < T_ - R_; ++k) {
+            const uint64_t b = 1ULL << round_->tglob[k];
+            if (m & b) r.thr |= 1u << k;
+            r.tile &= ~b;
+        }
+        return r;
+    }
+    std::string ctl_pred(const KOp& o, const std::string& base) {
+        const Split m = split_mask(o.cthr);
+        std::string p;
+        if (m.tile) {
+            std::string t = R64();
+            p = P();
+            I(fmt("and.b64 %s, %s, %llu", t.c_str(), base.c_str(), static_cast<unsigned long long>(m.tile)));
+            I(fmt("setp.eq.u64 %s, %s, %llu", p.c_str(), t.c_str(), static_cast<unsigned long long>(m.tile)));
+        }
+        if (m.thr) {
+            std::string t = R32(), q = P();
+            I(fmt("and.b32 %s, %s, %u", t.c_str(), tid_.c_str(), m.thr));
+            if (p.empty()) I(fmt("setp.eq.u32 %s, %s, %u", q.c_str(), t.c_str(), m.thr));
+            else I(fmt("setp.eq.and.u32 %s, %s, %u, %s", q.c_str(), t.c_str(), m.thr, p.c_str()));
+            p = q;
+        }
         return p;
     }
-    std::string par_pred(const KOp& o, const std::string& gthr) {
-        std::string t = R64(), c = R32(), c1 = R32(), p = P();
-        I(fmt("and.b64 %s, %s, %llu", t.c_str(), gthr.c_str(), static_cast<unsigned long long>(o.pthr)));
-        I(fmt("popc.b64 %s, %s", c.c_str(), t.c_str()));
+    std::string par_pred(const KOp& o, const std::string& base) {
+        const Split m = split_mask(o.pthr);
+        std::string v;
+        if (m.tile) {
+            std::string t = R64(), lo = R32(), hi = R32();
+            v = R32();
+            I(fmt("and.b64 %s, %s, %llu", t.c_str(), base.c_str(), static_cast<unsigned long long>(m.tile)));
+            I(fmt("mov.b64 {%s, %s}, %s", lo.c_str(), hi.c_str(), t.c_str()));
+            I(fmt("xor.b32 %s, %s, %s", v.c_str(), lo.c_str(), hi.c_str()));  // the parity of both words
+        }
+        std::string c = R32(), c1 = R32(), p = P();
+        if (m.thr) {
+            // the tile's parity joins as one more bit of the popcount's sum
+            std::string t = R32(), ct = R32();
+            I(fmt("and.b32 %s, %s, %u", t.c_str(), tid_.c_str(), m.thr));
+            I(fmt("popc.b32 %s, %s", ct.c_str(), t.c_str()));
+            if (v.empty()) {
+                c = ct;
+            } else {
+                std::string cv = R32();
+                I(fmt("popc.b32 %s, %s", cv.c_str(), v.c_str()));
+                I(fmt("add.u32 %s, %s, %s", c.c_str(), ct.c_str(), cv.c_str()));
+            }
+        } else {
+            I(fmt("popc.b32 %s, %s", c.c_str(), v.c_str()));
+        }
         I(fmt("and.b32 %s, %s, 1", c1.c_str(), c.c_str()));
         I(fmt("setp.ne.u32 %s, %s, 0", p.c_str(), c1.c_str()));
         return p;
     }
 
-    Cx phase(const Cx& a, const std::string& dr, const std::string& di, const std::string& ndi) {
-        // amp_phase: a * (dr + i di)
-        return {dot({{dr, a.x}, {ndi, a.y}}), dot({{dr, a.y}, {di, a.x}})};
+    Cx phase(Cx& a, const Cx& d) {  // amp_phase: a * (d.x + i d.y)
+        return lin({{d.x, &a, 0}, {d.y, &a, 1}});
     }
-    Cx special(const Cx& a, int sp) {  // amp_special: * -1, * i, * -i
-        if (sp == SP_NEG1) return {neg(a.x), neg(a.y)};
+    Cx special(Cx& a, int sp) {  // amp_special: * -1, * i, * -i
+        if (sp == SP_NEG1) return cneg(a);
+        xy(a);
         if (sp == SP_I) return {neg(a.y), a.x};
         return {a.y, neg(a.x)};
     }
@@ -1153,7 +1507,8 @@ class Gen {
         if (sp == SP_I) return {cnst(0.0), cnst(1.0)};
         return {cnst(0.0), cnst(-1.0)};
     }
-    Cx rot_q(const Cx& a, const std::string& s1, const std::string& s2) {  // a * i^q, q = s1 + 2 s2
+    Cx rot_q(Cx& a, const std::string& s1, const std::string& s2) {  // a * i^q, q = s1 + 2 s2
+        xy(a);
         Cx t{sel(neg(a.y), a.x, s1), sel(a.x, a.y, s1)};
         return {sel(neg(t.x), t.x, s2), sel(neg(t.y), t.y, s2)};
     }
@@ -1174,9 +1529,9 @@ class Gen {
         *d1 = (o.flags & F_D1_SPEC) ? special_value(o.special) : Cx{c[2], c[3]};
     }
 
-    void op_diag(const KOp& o, const std::string& gthr, const std::string& ctl) {
+    void op_diag(const KOp& o, const std::string& base, const std::string& ctl) {
         const bool tpar = (o.flags & F_TPAR) != 0;
-        std::string pt = tpar ? par_pred(o, gthr) : "";
+        std::string pt = tpar ? par_pred(o, base) : "";
         if (o.flags & F_UNIFORM) {
             if (!tpar) {
                 if (o.flags & F_D0_ONE) return;
@@ -1217,11 +1572,11 @@ class Gen {
                     for (int s = 0; s < NS_; ++s) {
                         if (h == 0) {
                             if (o.flags & F_D0_ONE) continue;
-                            A_[s][j] = phase(A_[s][j], c[0], c[1], neg(c[1]));
+                            A_[s][j] = phase(A_[s][j], {c[0], c[1]});
                         } else if (o.flags & F_D1_SPEC) {
                             A_[s][j] = special(A_[s][j], o.special);
                         } else {
-                            A_[s][j] = phase(A_[s][j], c[2], c[3], neg(c[3]));
+                            A_[s][j] = phase(A_[s][j], {c[2], c[3]});
                         }
                     }
                 }
@@ -1229,10 +1584,9 @@ class Gen {
                 Cx d0, d1;
                 diag_entries(o, &d0, &d1);
                 Cx f[2] = {{sel(d1.x, d0.x, pt), sel(d1.y, d0.y, pt)}, {sel(d0.x, d1.x, pt), sel(d0.y, d1.y, pt)}};
-                std::string nf[2] = {neg(f[0].y), neg(f[1].y)};
                 for (int j = 0; j < NA_; ++j) {
                     const int h = (j >> t) & 1;
-                    for (int s = 0; s < NS_; ++s) A_[s][j] = phase(A_[s][j], f[h].x, f[h].y, nf[h]);
+                    for (int s = 0; s < NS_; ++s) A_[s][j] = phase(A_[s][j], f[h]);
                 }
             }
         } else {
@@ -1246,11 +1600,11 @@ class Gen {
                 f[0] = {sel(d1.x, d0.x, pt), sel(d1.y, d0.y, pt)};
                 f[1] = {sel(d0.x, d1.x, pt), sel(d0.y, d1.y, pt)};
             }
-            std::string nf[2] = {neg(f[0].y), neg(f[1].y)};
             for (int j = 0; j < NA_; ++j) {
                 if ((static_cast<uint32_t>(j) & o.creg) != o.creg) continue;
                 const int par = __builtin_popcount(static_cast<uint32_t>(j) & o.preg) & 1;
-                for (int s = 0; s < NS_; ++s) A_[s][j] = phase(A_[s][j], f[par].x, f[par].y, nf[par]);
+                if (par == 0 && !tpar && (o.flags & F_D0_ONE)) continue;
+                for (int s = 0; s < NS_; ++s) A_[s][j] = phase(A_[s][j], f[par]);
             }
         }
         guard(old, ctl);
@@ -1270,8 +1624,7 @@ class Gen {
             // each entry's coefficients just before their use (a table of 2^R
             // entries loaded at once would hold 2^(R+1) registers)
             const std::vector<std::string> c = coefs(o.coef + 2 * j, 2);
-            const std::string dr = c[0], di = c[1], ndi = neg(di);
-            for (int s = 0; s < NS_; ++s) A_[s][j] = phase(A_[s][j], dr, di, ndi);
+            for (int s = 0; s < NS_; ++s) A_[s][j] = phase(A_[s][j], {c[0], c[1]});
         }
     }
 
@@ -1282,7 +1635,8 @@ class Gen {
             n = f;
             if (!ctl.empty()) n = {sel(f.x, cnst(1.0), ctl), sel(f.y, cnst(0.0), ctl)};
         } else {
-            n = phase(ph_, f.x, f.y, neg(f.y));
+            n = phase(ph_, f);
+            xy(n);
             if (!ctl.empty()) n = {sel(n.x, ph_.x, ctl), sel(n.y, ph_.y, ctl)};
         }
         ph_ = n;
@@ -1290,12 +1644,11 @@ class Gen {
     }
 
     // thread-controlled op: keep the old values where the control is 0
-    void guard(const std::vector<std::vector<Cx>>& old, const std::string& ctl) {
+    void guard(std::vector<std::vector<Cx>>& old, const std::string& ctl) {
         if (ctl.empty()) return;
         for (int s = 0; s < NS_; ++s)
             for (int j = 0; j < NA_; ++j)
-                if (!same(A_[s][j], old[s][j]))
-                    A_[s][j] = {sel(A_[s][j].x, old[s][j].x, ctl), sel(A_[s][j].y, old[s][j].y, ctl)};
+                if (!same(A_[s][j], old[s][j])) A_[s][j] = csel(A_[s][j], old[s][j], ctl);
     }
 
     void op_gate(const KOp& o, const std::string& ctl) {
@@ -1309,7 +1662,9 @@ class Gen {
             case K_Y:
                 for (int j : pairs(t, o.creg))
                     for (int s = 0; s < NS_; ++s) {
-                        const Cx a = A_[s][j], b = A_[s][j | (1 << t)];
+                        Cx a = A_[s][j], b = A_[s][j | (1 << t)];
+                        xy(a);
+                        xy(b);
                         A_[s][j] = {b.y, neg(b.x)};
                         A_[s][j | (1 << t)] = {neg(a.y), a.x};
                     }
@@ -1317,33 +1672,37 @@ class Gen {
             case K_HAD:
                 for (int j : pairs(t, o.creg))
                     for (int s = 0; s < NS_; ++s) {
-                        const Cx a = A_[s][j], b = A_[s][j | (1 << t)];
-                        A_[s][j] = {add(a.x, b.x), add(a.y, b.y)};
-                        A_[s][j | (1 << t)] = {sub(a.x, b.x), sub(a.y, b.y)};
+                        Cx a = A_[s][j], b = A_[s][j | (1 << t)];
+                        A_[s][j] = cadd(a, b);
+                        A_[s][j | (1 << t)] = csub(a, b);
+                        // where the thread's bit t is flipped, a and b are exchanged:
+                        // the same sum, the difference's sign; nothing stays flipped
+                        if (!flip_[t].empty()) A_[s][j | (1 << t)] = cneg_if(A_[s][j | (1 << t)], flip_[t]);
                     }
+                flip_[t].clear();
                 break;
             case K_REAL: {
                 std::vector<std::string> m = coefs(o.coef, 4);
                 if (!flip_[t].empty()) {  // X U X = [[m3, m2], [m1, m0]] where the thread's bit t is flipped
                     const std::string& p = flip_[t];
-                    m = {sel(m[3], m[0], p), sel(m[2], m[1], p), sel(m[1], m[2], p), sel(m[0], m[3], p)};
+                    const std::vector<std::string> c = m;
+                    m = {sel(c[3], c[0], p), sel(c[2], c[1], p), sel(c[1], c[2], p), sel(c[0], c[3], p)};
                 }
                 for (int j : pairs(t, o.creg))
                     for (int s = 0; s < NS_; ++s) {
-                        const Cx a = A_[s][j], b = A_[s][j | (1 << t)];
-                        A_[s][j] = {dot({{m[0], a.x}, {m[1], b.x}}), dot({{m[0], a.y}, {m[1], b.y}})};
-                        A_[s][j | (1 << t)] = {dot({{m[2], a.x}, {m[3], b.x}}), dot({{m[2], a.y}, {m[3], b.y}})};
+                        Cx a = A_[s][j], b = A_[s][j | (1 << t)];
+                        A_[s][j] = lin({{m[0], &a, 0}, {m[1], &b, 0}});
+                        A_[s][j | (1 << t)] = lin({{m[2], &a, 0}, {m[3], &b, 0}});
                     }
                 break;
             }
             case K_RX: {
-                std::vector<std::string> m = coefs(o.coef, 2);
-                const std::string c = m[0], sn = m[1], ns = neg(m[1]);
+                const std::vector<std::string> m = coefs(o.coef, 2);
                 for (int j : pairs(t, o.creg))
                     for (int s = 0; s < NS_; ++s) {
-                        const Cx a = A_[s][j], b = A_[s][j | (1 << t)];
-                        A_[s][j] = {dot({{c, a.x}, {sn, b.y}}), dot({{c, a.y}, {ns, b.x}})};
-                        A_[s][j | (1 << t)] = {dot({{c, b.x}, {sn, a.y}}), dot({{c, b.y}, {ns, a.x}})};
+                        Cx a = A_[s][j], b = A_[s][j | (1 << t)];
+                        A_[s][j] = lin({{m[0], &a, 0}, {m[1], &b, 3}});
+                        A_[s][j | (1 << t)] = lin({{m[0], &b, 0}, {m[1], &a, 3}});
                     }
                 break;
             }
@@ -1356,15 +1715,11 @@ class Gen {
                         for (int c = 0; c < 2; ++c) f[2 * e + c] = sel(m[2 * (3 - e) + c], m[2 * e + c], p);
                     m = f;
                 }
-                std::string nmi[4];
-                for (int i = 0; i < 4; ++i) nmi[i] = neg(m[2 * i + 1]);
                 for (int j : pairs(t, o.creg))
                     for (int s = 0; s < NS_; ++s) {
-                        const Cx a = A_[s][j], b = A_[s][j | (1 << t)];
-                        A_[s][j] = {dot({{m[0], a.x}, {nmi[0], a.y}, {m[2], b.x}, {nmi[1], b.y}}),
-                                    dot({{m[0], a.y}, {m[1], a.x}, {m[2], b.y}, {m[3], b.x}})};
-                        A_[s][j | (1 << t)] = {dot({{m[4], a.x}, {nmi[2], a.y}, {m[6], b.x}, {nmi[3], b.y}}),
-                                               dot({{m[4], a.y}, {m[5], a.x}, {m[6], b.y}, {m[7], b.x}})};
+                        Cx a = A_[s][j], b = A_[s][j | (1 << t)];
+                        A_[s][j] = lin({{m[0], &a, 0}, {m[1], &a, 1}, {m[2], &b, 0}, {m[3], &b, 1}});
+                        A_[s][j | (1 << t)] = lin({{m[4], &a, 0}, {m[5], &a, 1}, {m[6], &b, 0}, {m[7], &b, 1}});
                     }
                 break;
             }
@@ -1383,50 +1738,118 @@ class Gen {
         guard(old, ctl);
     }
 
+    // sum over a probe's registers of the real (or imaginary) part of
+    // conj(lam_j) psi_jx, jx = j ^ xreg, with the sign of jx's Z bits
+    std::string probe_f64(const KOp& o, bool im) {
+        std::vector<std::pair<std::string, bool>> t;
+        for (int j : probe_regs(o)) {
+            const int jx = j ^ static_cast<int>(o.xreg);
+            const Cx l = A_[1][j], w = A_[0][jx];
+            t.push_back({im ? fma(l.x, w.y, neg(mul(l.y, w.x))) : fma(l.x, w.x, mul(l.y, w.y)), probe_sign(o, jx)});
+        }
+        return signed_tree(t);
+    }
+    std::vector<int> probe_regs(const KOp& o) const {
+        std::vector<int> r;
+        for (int j = 0; j < NA_; ++j)
+            if ((static_cast<uint32_t>(j) & o.creg) == o.creg) r.push_back(j);
+        return r;
+    }
+    static bool probe_sign(const KOp& o, int jx) {
+        return (__builtin_popcount(static_cast<uint32_t>(jx) & o.preg) & 1) != 0;
+    }
+    // balanced tree over (value, negated) terms
+    std::string signed_tree(std::vector<std::pair<std::string, bool>> t) {
+        if (t.empty()) return cnst(0.0);
+        while (t.size() > 1) {
+            std::vector<std::pair<std::string, bool>> n;
+            for (size_t i = 0; i + 1 < t.size(); i += 2) {
+                const auto &a = t[i], &b = t[i + 1];
+                if (a.second == b.second) n.push_back({add(a.first, b.first), a.second});
+                else if (a.second) n.push_back({sub(b.first, a.first), false});
+                else n.push_back({sub(a.first, b.first), false});
+            }
+            if (t.size() & 1) n.push_back(t.back());
+            t.swap(n);
+        }
+        return t[0].second ? neg(t[0].first) : t[0].first;
+    }
+    // Complex64: per sign, products in runs of four FMAs whose sums meet in a
+    // tree.  Real part: l and w packed, the two halves added at the end.
+    // Imaginary part: l.x w.y and l.y w.x on the real registers.
+    std::string probe_f32(const KOp& o, bool im) {
+        std::vector<std::pair<std::string, bool>> t;
+        std::string run[2][2];
+        int len[2] = {0, 0};
+        auto close = [&](int g) {
+            if (len[g] == 0) return;
+            if (im) {
+                t.push_back({f32op("sub", run[g][0], run[g][1]), g == 1});
+            } else {
+                auto [x, y] = split(run[g][0]);
+                t.push_back({f32op("add", x, y), g == 1});
+            }
+            len[g] = 0;
+        };
+        for (int j : probe_regs(o)) {
+            const int jx = j ^ static_cast<int>(o.xreg);
+            const int g = probe_sign(o, jx) ? 1 : 0;
+            Cx &l = A_[1][j], &w = A_[0][jx];
+            if (im) {
+                xy(l);
+                xy(w);
+                run[g][0] = len[g] ? f32fma(l.x, w.y, run[g][0]) : f32op("mul", l.x, w.y);
+                run[g][1] = len[g] ? f32fma(l.y, w.x, run[g][1]) : f32op("mul", l.y, w.x);
+            } else {
+                run[g][0] = len[g] ? q2fma(pk(l), pk(w), run[g][0]) : q2("mul", pk(l), pk(w));
+            }
+            if (++len[g] == 4) close(g);
+        }
+        close(0);
+        close(1);
+        return signed_tree(t);
+    }
+    // Double-single: l and w (turned by -i for the imaginary part: then the
+    // halves are l.x w.y and -l.y w.x) multiplied packed, one running pair
+    // per sign, the halves added at the end.
+    std::string probe_ds(const KOp& o, bool im) {
+        std::string s[2], e[2];
+        for (int j : probe_regs(o)) {
+            const int jx = j ^ static_cast<int>(o.xreg);
+            const int g = probe_sign(o, jx) ? 1 : 0;
+            Cx &l = A_[1][j], &w = A_[0][jx];
+            const std::string lp = pk(l), wp = pk(turned(w, im ? 3 : 0));
+            if (s[g].empty()) {
+                auto [lh, ll] = hl(lp);
+                auto [wh, wl] = hl(wp);
+                const std::string p = q2mul(lh, wh);
+                s[g] = p;
+                e[g] = q2fma(ll, wh, q2fma(lh, wl, q2fma(lh, wh, q2("sub", zero2_, p))));
+            } else {
+                ds_axpy(lp, wp, &s[g], &e[g]);
+            }
+        }
+        std::vector<std::pair<std::string, bool>> t;
+        for (int g = 0; g < 2; ++g) {
+            if (s[g].empty()) continue;
+            auto [xh, yh] = split(s[g]);
+            auto [xl, yl] = split(e[g]);
+            t.push_back({ds_add(xh + "|" + xl, yh + "|" + yl), g == 1});
+        }
+        return signed_tree(t);
+    }
+
     // Im<lam| Q |psi> share of the thread (probe_sum / reg_probe of
     // adjoint.cuh, the register terms summed as a balanced tree).  The
     // thread values of up to 8 probes wait in registers and are warp-summed
     // together (flush_probes).
-    void op_probe(const KOp& o, const std::string& gthr, const std::string& ctl) {
-        struct Term {
-            std::string r;
-            bool neg;
-        };
-        std::vector<Term> tr, ti;
-        for (int j = 0; j < NA_; ++j) {
-            if ((static_cast<uint32_t>(j) & o.creg) != o.creg) continue;
-            const int jx = j ^ static_cast<int>(o.xreg);
-            const bool ng = (__builtin_popcount(static_cast<uint32_t>(jx) & o.preg) & 1) != 0;
-            const Cx l = A_[1][j], w = A_[0][jx];
-            tr.push_back({fma(l.x, w.x, mul(l.y, w.y)), ng});
-            ti.push_back({fma(l.x, w.y, neg(mul(l.y, w.x))), ng});
-        }
-        auto tree = [&](std::vector<Term> t) -> std::string {
-            if (t.empty()) return cnst(0.0);
-            while (t.size() > 1) {
-                std::vector<Term> n;
-                for (size_t i = 0; i + 1 < t.size(); i += 2) {
-                    const Term& a = t[i];
-                    const Term& b = t[i + 1];
-                    if (a.neg == b.neg) n.push_back({add(a.r, b.r), a.neg});
-                    else if (a.neg) n.push_back({sub(b.r, a.r), false});
-                    else n.push_back({sub(a.r, b.r), false});
-                }
-                if (t.size() & 1) n.push_back(t.back());
-                t.swap(n);
-            }
-            return t[0].neg ? neg(t[0].r) : t[0].r;
-        };
-        const std::string ar = tree(tr), ai = tree(ti);
+    void op_probe(const KOp& o, const std::string& base, const std::string& ctl) {
+        const bool im = (o.special & 1) == 0;  // needs the imaginary part of sum conj(l) w (else the real part)
+        const std::string sum = f64_ ? probe_f64(o, im) : (ds_ ? probe_ds(o, im) : probe_f32(o, im));
         std::string v;
-        switch (o.special & 3) {
-            case 0: v = ai; break;
-            case 1: v = ar; break;
-            case 2: v = neg(ai); break;
-            default: v = neg(ar); break;
-        }
+        v = (o.special & 2) ? neg(sum) : sum;
         if (o.flags & F_TPAR) {
-            std::string pt = par_pred(o, gthr);
+            std::string pt = par_pred(o, base);
             v = sel(neg(v), v, pt);
         }
         if (!ctl.empty()) v = sel(v, cnst(0.0), ctl);
@@ -1561,8 +1984,6 @@ class Gen {
                 I(fmt("@%s bra %s", p.c_str(), lskip.c_str()));
             }
             const std::vector<std::string> m = coefs(o.coef, 32);
-            std::vector<std::string> nm(16);
-            for (int e = 0; e < 16; ++e) nm[e] = neg(m[2 * e + 1]);
             const int lo = o.t0 < o.t1 ? o.t0 : o.t1, hi = o.t0 < o.t1 ? o.t1 : o.t0;
             const uint32_t d0 = tile_weight(o.t0, padu_) * es_, d1 = tile_weight(o.t1, padu_) * es_;
             const int iters = (1 << (T_ - 2)) / NT_;
@@ -1603,16 +2024,12 @@ class Gen {
                     Cx out[4];
                     for (int r = 0; r < 4; ++r) {  // quad_dense of policy.cuh
                         const int b0 = 8 * r;
-                        std::vector<std::pair<std::string, std::string>> tr, ti;
+                        std::vector<Term> t;
                         for (int c = 0; c < 4; ++c) {
-                            const std::string& mr = m[b0 + 2 * c];
-                            const std::string& mi = m[b0 + 2 * c + 1];
-                            tr.push_back({mr, in[c].x});
-                            tr.push_back({nm[4 * r + c], in[c].y});
-                            ti.push_back({mr, in[c].y});
-                            ti.push_back({mi, in[c].x});
+                            t.push_back({m[b0 + 2 * c], &in[c], 0});
+                            t.push_back({m[b0 + 2 * c + 1], &in[c], 1});
                         }
-                        out[r] = {dot(tr), dot(ti)};
+                        out[r] = lin(t);
                     }
                     for (int v = 0; v < 4; ++v) store_amp(ad, st * tileB_ + dx[v], out[v], pc);
                 }
@@ -1623,9 +2040,7 @@ class Gen {
     }
 
     void round(const StepDesc& sd, const std::string& base, const std::string& sbase) {
-        bool need_g = false;
-        for (int oi = 0; oi < sd.op_count; ++oi)
-            if (hp_.ops[sd.op_begin + oi].flags & (F_TCTRL | F_TPAR)) need_g = true;
+        round_ = &sd;
         // the thread's tile-layout byte address in this slot; register j adds offb(j)
         std::vector<uint32_t> tsw(T_ - R_);
         for (int k = 0; k < T_ - R_; ++k) tsw[k] = static_cast<uint32_t>(sd.tsw[k]) * es_;
@@ -1637,14 +2052,6 @@ class Gen {
         if (es_ == 8)
             for (int k = 0; k < R_; ++k)
                 if (sd.rpos[k] == 0) r0 = k;
-        std::string gthr;
-        if (need_g) {
-            std::vector<uint64_t> tg(T_ - R_);
-            for (int k = 0; k < T_ - R_; ++k) tg[k] = 1ULL << sd.tglob[k];
-            std::string td = deposit64(tid_, T_ - R_, tg);
-            gthr = R64();
-            I(fmt("or.b64 %s, %s, %s", gthr.c_str(), base.c_str(), td.c_str()));
-        }
         auto offb = [&](int j) {
             uint32_t o = 0;
             for (int k = 0; k < R_; ++k)
@@ -1658,11 +2065,11 @@ class Gen {
                 if ((j >> r0) & 1) continue;
                 const int j1 = j | (1 << r0);
                 for (int s = 0; s < NS_; ++s) {
-                    Cx a{A(), A()}, b{A(), A()};
-                    I(fmt("ld.shared.v4.f32 {%s, %s, %s, %s}, [%s+%u]", a.x.c_str(), a.y.c_str(), b.x.c_str(),
-                          b.y.c_str(), psb.c_str(), s * tileB_ + offb(j)));
-                    A_[s][j] = a;
-                    A_[s][j1] = b;
+                    std::string a = Q(), b = Q();
+                    I(fmt("ld.shared.v2.b64 {%s, %s}, [%s+%u]", a.c_str(), b.c_str(), psb.c_str(),
+                          s * tileB_ + offb(j)));
+                    A_[s][j] = Cx::packed(a);
+                    A_[s][j1] = Cx::packed(b);
                 }
                 continue;
             }
@@ -1673,7 +2080,7 @@ class Gen {
         flip_.assign(R_, std::string());
         for (int oi = 0; oi < sd.op_count; ++oi) {
             const KOp& o = hp_.ops[sd.op_begin + oi];
-            const std::string ctl = (o.flags & F_TCTRL) ? ctl_pred(o, gthr) : "";
+            const std::string ctl = (o.flags & F_TCTRL) ? ctl_pred(o, base) : "";
             if (o.kind == K_X && !ctl.empty() && o.creg == 0) {
                 add_flip(o.t0, ctl);  // thread-controlled X: a pending flip of the thread's bit t0
                 continue;
@@ -1681,18 +2088,18 @@ class Gen {
             // register controls, parities and targets whose meaning a flip changes
             uint32_t need = o.creg;
             if (o.kind == K_DIAG) need |= o.preg | ((o.flags & F_ONEBIT) ? (1u << o.t0) : 0u);
-            if (o.kind == K_Y || o.kind == K_HAD) need |= 1u << o.t0;
+            if (o.kind == K_Y || (o.kind == K_HAD && o.creg)) need |= 1u << o.t0;
             if (o.kind == K_SWAP && o.creg) need |= (1u << o.t0) | (1u << o.t1);
             if (o.kind == K_PROBE) need |= o.xreg | o.preg;
-            if (o.kind == K_DIAGR) need |= (1u << R_) - 1;  // its entries are per register index
+            if (o.kind == K_DIAGR) need |= o.xreg;  // the register bits its entries depend on
             for (int t = 0; t < R_; ++t)
                 if ((need >> t) & 1) {
                     if (!flip_[t].empty()) note(fmt("materialize flip %d for kind %d", t, o.kind));
                     materialize(t);
                 }
             note(fmt("op kind %d t0 %d%s", o.kind, o.t0, ctl.empty() ? "" : " thread-controlled"));
-            if (o.kind == K_PROBE) op_probe(o, gthr, ctl);
-            else if (o.kind == K_DIAG) op_diag(o, gthr, ctl);
+            if (o.kind == K_PROBE) op_probe(o, base, ctl);
+            else if (o.kind == K_DIAG) op_diag(o, base, ctl);
             else if (o.kind == K_DIAGR) op_diagr(o);
             else op_gate(o, ctl);
         }
@@ -1712,11 +2119,9 @@ class Gen {
                     for (int j = 0; j < NA_; ++j) A_[s][j] = rot_q(A_[s][j], s1, s2);
             }
         }
-        if (ph_on_) {
-            const std::string nfi = neg(ph_.y);
+        if (ph_on_)
             for (int s = 0; s < NS_; ++s)
-                for (int j = 0; j < NA_; ++j) A_[s][j] = phase(A_[s][j], ph_.x, ph_.y, nfi);
-        }
+                for (int j = 0; j < NA_; ++j) A_[s][j] = phase(A_[s][j], ph_);
         // a pending flip of bit t: register j holds logical j ^ (1 << t), whose
         // address is j's plus rsw[t] (bit t of j clear) or minus it (set)
         if (r0 >= 0) materialize(r0);  // pairs are stored as they are
@@ -1753,8 +2158,8 @@ class Gen {
                 const int j1 = j | (1 << r0);
                 const std::string ad = store_base(j);
                 for (int s = 0; s < NS_; ++s)
-                    I(fmt("st.shared.v4.f32 [%s+%u], {%s, %s, %s, %s}", ad.c_str(), s * tileB_ + offb(j),
-                          A_[s][j].x.c_str(), A_[s][j].y.c_str(), A_[s][j1].x.c_str(), A_[s][j1].y.c_str()));
+                    I(fmt("st.shared.v2.b64 [%s+%u], {%s, %s}", ad.c_str(), s * tileB_ + offb(j),
+                          pk(A_[s][j]).c_str(), pk(A_[s][j1]).c_str()));
                 continue;
             }
             const std::string ad = store_base(j);
@@ -1779,9 +2184,9 @@ class Gen {
         flip_[t].clear();
         for (int j : pairs(t, 0))
             for (int s = 0; s < NS_; ++s) {
-                const Cx a = A_[s][j], b = A_[s][j | (1 << t)];
-                A_[s][j] = {sel(b.x, a.x, p), sel(b.y, a.y, p)};
-                A_[s][j | (1 << t)] = {sel(a.x, b.x, p), sel(a.y, b.y, p)};
+                Cx a = A_[s][j], b = A_[s][j | (1 << t)];
+                A_[s][j] = csel(b, a, p);
+                A_[s][j | (1 << t)] = csel(a, b, p);
             }
     }
 
@@ -1798,13 +2203,20 @@ class Gen {
     bool bulk_out_ = true;                     // write-back by bulk stores of the slot
     std::string smend_, gend_[2];
     bool pc_ = false;  // coefficients from the parameter block p_cblob
-    uint32_t cmin_ = 0, cmax_ = 0;
-    static constexpr uint32_t kMaxBlob = 16384;  // bytes of coefficients in the kernel parameters
+    std::vector<uint32_t> clist_;            // pool entries of the parameter block
+    std::map<uint32_t, uint32_t> cindex_;    // pool entry -> its place there
+    static constexpr uint32_t kMaxBlob = 24576;  // bytes of coefficients in the kernel parameters
+    uint32_t pb_;                                // bytes of one of them
+    std::map<std::string, std::string> both_, negc_;
+    std::map<std::string, uint32_t> param_at_;  // parameter-block offset of a coefficient
+    std::map<std::string, Cx> turned_;
+    std::map<std::string, std::string> sign_;  // predicate -> sign-bit mask of a packed register
     std::string body_;
-    int nr_ = 0, nrd_ = 0, nh_ = 0, np_reg_ = 0, na_ = 0, nd_ = 0, nl_ = 0;
+    int nr_ = 0, nrd_ = 0, nh_ = 0, np_reg_ = 0, na_ = 0, nd_ = 0, nq_ = 0, nl_ = 0;
     std::map<double, std::string> consts_;
     std::string tid_, bid64_, nbid64_, stg_[2], ntiles_, coef0_, cstrideB_, ishift_, active_, hasact_, smb_;
     std::string gtidB_, stidB_, lane_, paccB_, paccW_, perTile_, partial_, coefp_;
+    std::string zero2_;  // a packed zero the assembler does not know (q2mul)
     std::string status_, waitns_, extra_, iss_, t0_, runG_, runS_, runb_, txb_, mbarB_;
     struct Pending {
         std::string v;
@@ -1814,6 +2226,7 @@ class Gen {
     std::vector<Pending> pending_;
     std::vector<std::vector<Cx>> A_;
     std::vector<std::string> flip_;
+    const StepDesc* round_ = nullptr;  // the round being emitted
     bool ph_on_ = false;
     Cx ph_;
     std::string q_;
@@ -1873,7 +2286,7 @@ bool jit_pass_key(const HostPlan& hp, int pi, const JitShape& sh, std::string* k
             put(&k, o.preg);
             put(&k, o.cthr);
             put(&k, o.pthr);
-            put(&k, o.coef);
+            if (!g.param_coefs()) put(&k, o.coef);  // the parameter block is numbered by use
             put(&k, o.xreg);
             put(&k, o.k);
             k.append(reinterpret_cast<const char*>(o.tk), sizeof o.tk);
@@ -1882,12 +2295,11 @@ bool jit_pass_key(const HostPlan& hp, int pi, const JitShape& sh, std::string* k
     return true;
 }
 
-bool jit_pass_coef_block(const HostPlan& hp, int pi, const JitShape& sh, uint32_t* cmin, uint32_t* cmax) {
+bool jit_pass_coef_block(const HostPlan& hp, int pi, const JitShape& sh, std::vector<uint32_t>* entries) {
     if (pi < 0 || pi >= static_cast<int>(hp.passes.size())) return false;
     Gen g(hp, pi, sh);
     if (!g.param_coefs()) return false;
-    *cmin = g.cmin();
-    *cmax = g.cmax();
+    *entries = g.coef_entries();
     return true;
 }
 

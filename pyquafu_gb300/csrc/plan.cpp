@@ -1095,6 +1095,7 @@ void merge_round_diagonals(HostPlan* plan) {
                     std::memset(&k, 0, sizeof(k));
                     k.kind = K_DIAGR;
                     k.k = static_cast<uint8_t>(R);
+                    k.xreg = support;
                     k.coef = static_cast<uint32_t>(plan->coef.size());
                     for (int j = 0; j < NA; ++j) {
                         plan->coef.push_back(table[j].real());

@@ -359,3 +359,32 @@ def test_largest_passes_fit_their_register_budget(precision, adjoint, spill_max)
             assert spill and int(spill[0]) <= spill_max, (i, log)
     finally:
         lib.qfvm_plan_destroy(h)
+
+
+@pytest.mark.parametrize("precision", [1, 2])
+def test_parameter_block_holds_what_a_pass_reads(precision):
+    """Merged diagonal tables sit behind the gates in a plan's pool; a pass's
+    parameter block lists only the entries it reads, so the default passes of
+    the 30-qubit circuit read every coefficient from it."""
+    h = default_plan(precision, False)
+    for i in (0, 20, 40):
+        src = pass_ptx(h, i, 1)
+        assert "p_cblob[" in src and "ld.global.nc" not in src
+    nat.load().qfvm_plan_destroy(h)
+
+
+def test_float_pair_products_are_rounded():
+    """Float-pair arithmetic needs every packed product rounded before it is
+    added: the assembler contracts mul.rn.f32x2 with a following packed add,
+    so those products are FMAs with the zero of the kernel parameters.  The
+    multiplications that remain only start chains of FMAs of low parts."""
+    import re
+
+    h = default_plan(2, False)
+    src = pass_ptx(h, 3, 1)
+    nat.load().qfvm_plan_destroy(h)
+    zero = re.search(r"ld\.param\.b64 (%q\d+), \[p_zero2\]", src).group(1)
+    assert re.search(rf"fma\.rn\.f32x2 %q\d+, %q\d+, %q\d+, {zero};", src)
+    for q in re.findall(r"mul\.rn\.f32x2 (%q\d+),", src):
+        uses = re.findall(rf"\n\t(\S+) %q\d+, [^;]*{q}[,;]", src)
+        assert uses and all(u == "fma.rn.f32x2" for u in uses), (q, uses)
