@@ -121,8 +121,7 @@ int make_plan(int n, int precision, const qfvm_op* ops, int64_t n_ops, const dou
     std::vector<GOp> gops;
     std::string err;
     if (!classify(n, ops, n_ops, matpool, matpool_len, &gops, &err)) return fail(QFVM_ERR_INVALID, err);
-    fuse_single_qubit(&gops);
-    unnormalize_hadamards(&gops);
+    simplify_plain(&gops);
     const int sp = store_precision(precision);
     if (T > 0 || R > 0) {
         int dT, dR;
@@ -144,6 +143,7 @@ int make_plan_gops(int n, int precision, const std::vector<GOp>& gops, int T, in
         delete p;
         return fail(QFVM_ERR_INVALID, err);
     }
+    normalize_passes(&p->hp);
     if (merge_diagonals) merge_round_diagonals(&p->hp);
     p->hp.arith = (precision == QFVM_C128_DS) ? QFVM_C128_DS : sp;
     int rc = upload_plan(p);
@@ -639,8 +639,7 @@ int qfvm_plan_host_build(int32_t num_qubits, int32_t precision, const qfvm_op* o
     std::vector<GOp> gops;
     std::string err;
     if (!classify(num_qubits, ops, n_ops, matpool, matpool_len, &gops, &err)) return fail(QFVM_ERR_INVALID, err);
-    fuse_single_qubit(&gops);
-    unnormalize_hadamards(&gops);
+    simplify_plain(&gops);
     if (tile_qubits > 0 || reg_qubits > 0) {
         int dT, dR;
         default_shape(num_qubits, store_precision(precision), &dT, &dR);
@@ -656,6 +655,7 @@ int qfvm_plan_host_build(int32_t num_qubits, int32_t precision, const qfvm_op* o
         return fail(QFVM_ERR_INVALID, err);
     }
     p->hp.arith = precision;
+    normalize_passes(&p->hp);
     merge_round_diagonals(&p->hp);
     *out = p;
     return QFVM_OK;
@@ -669,6 +669,7 @@ int qfvm_plan_host_build_adjoint(int32_t num_qubits, int32_t precision, const qf
     std::string err;
     if (!classify(num_qubits, ops, n_ops, matpool, matpool_len, &gops, &err)) return fail(QFVM_ERR_INVALID, err);
     if (!build_adjoint_sweep(gops, &sweep, &err)) return fail(QFVM_ERR_INVALID, err);
+    for (GOp& g : sweep) g.bkind = 0;
     int aT = 0, aR = 0;
     resolve_shape(precision, 1, num_qubits, &aT, &aR);
     qfvm_plan* p = new qfvm_plan();
@@ -677,6 +678,7 @@ int qfvm_plan_host_build_adjoint(int32_t num_qubits, int32_t precision, const qf
         return fail(QFVM_ERR_INVALID, err);
     }
     p->hp.arith = precision;
+    normalize_passes(&p->hp);
     *out = p;
     return QFVM_OK;
 }
@@ -845,15 +847,17 @@ int qfvm_adjoint(int32_t num_qubits, int32_t precision, const qfvm_op* ops, int6
         if (g.slot >= n_slots) return fail(QFVM_ERR_INVALID, "parameter slot beyond n_slots");
     std::vector<GOp> sweep;
     if (!build_adjoint_sweep(gops, &sweep, &err)) return fail(QFVM_ERR_INVALID, err);
+    for (GOp& g : sweep) g.bkind = 0;  // planned at these angles: nothing is bound later
     for (const GOp& g : sweep)
         if (g.kind == K_PROBE && __builtin_popcountll(g.xmask) > 2)
             return fail(QFVM_ERR_UNSUPPORTED, "generators flipping more than two qubits are not supported");
     const int storage = store_precision(precision);
     const int arith = precision;
 
-    // forward pass on psi
+    // forward pass on psi: a plain simulation
     qfvm_plan* fwd = nullptr;
-    QSV_TRY(make_plan_gops(n, precision, gops, 0, 0, &fwd));
+    simplify_plain(&gops);
+    QSV_TRY(make_plan_gops(n, precision, gops, 0, 0, &fwd, true));
     int aT = 0, aR = 0;
     resolve_shape(arith, 1, n, &aT, &aR);
     qfvm_plan* rev = nullptr;

@@ -46,6 +46,8 @@ enum : uint8_t {
     F_TPAR = 32     // register round: pthr != 0 (a parity or Z bit on a thread bit)
 };
 enum : uint8_t { SP_NEG1 = 1, SP_I = 2, SP_NEGI = 3 };
+// K_REAL / K_RX `special`: both diagonal entries are exactly 1 (normalize_passes)
+enum : uint8_t { SP_UNIT = 1 };
 
 constexpr int MAXK = 6;  // largest dense target count held in a thread's registers (k_globalop, k_small)
 // Dense gates on MAXK+1 .. MAX_DENSE_TARGETS targets run one CTA per group of
@@ -244,6 +246,9 @@ void unnormalize_hadamards(std::vector<GOp>* gops);
 // the qubit only as a control; X-type gates pass X / RX on the same target):
 // d.d' -> one diagonal, rx(a) rx(b) -> rx(a + b), X X -> nothing.
 void fuse_single_qubit(std::vector<GOp>* gops);
+// Plain simulation plans (no probes, nothing bound per item): parameter slots
+// dropped, then the two rewrites above.
+void simplify_plain(std::vector<GOp>* gops);
 // Plain simulation plans: inside every register round of at most 4 register
 // qubits, diagonal ops whose parity and controls are all register bits are
 // multiplied into one per-register-entry phase table (K_DIAGR), applied
@@ -252,6 +257,13 @@ void fuse_single_qubit(std::vector<GOp>* gops);
 // between their places and that point.  Entries that come out exactly 1,
 // -1, i or -i are coded so the kernels apply them without arithmetic.
 void merge_round_diagonals(HostPlan* plan);
+// Plans without binds: inside every tile pass, uncontrolled rotations
+// [[c, -s], [s, c]] and [[c, -is], [-is, c]] become c * (1 on the diagonal)
+// and register-bit phases d0 * diag(1, d1 / d0); the scalars' product, which
+// commutes with everything, goes back into one gate of the pass.  A rotation
+// then costs one multiply-add per real instead of a multiply and a
+// multiply-add, a phase half the amplitudes.  Probes are rescaled to match.
+void normalize_passes(HostPlan* plan);
 // Coefficients of a bindable gate kind at angle th (2 or 4 doubles).
 int bind_coef(int kind, double th, double* c);
 // Gate-equivalent bytes of one gop: 2 * bytes per amplitude * amplitudes it

@@ -23,7 +23,9 @@
 // operands of the arithmetic itself.  Measured on the benchmark family,
 // scalar arithmetic and coefficients mostly loaded per thread before:
 // 30 qubits float pairs 1057 -> 939 ms, 27 qubits complex64 20.4 -> 18.2 ms,
-// 24-qubit float-pair gradient 133 -> 101 ms.
+// 24-qubit float-pair gradient 133 -> 101 ms.  With the unit rotations of
+// normalize_passes: 827 ms, 16.5 ms (0.81 of the measured copy bandwidth)
+// and 85 ms; 25 qubits FP64 (bound by the FP64 pipe) 88.0 -> 55.3 ms.
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -126,6 +128,8 @@ class Gen {
                 }
                 for (int i = 0; i < n; ++i) {
                     if (o.kind == K_DIAGR && diagr_code(o, i / 2) != DIAGR_GENERAL) continue;
+                    if (o.special == SP_UNIT && ((o.kind == K_REAL && (i == 0 || i == 3)) || (o.kind == K_RX && i == 0)))
+                        continue;
                     const uint32_t at = o.coef + static_cast<uint32_t>(i);
                     if (cindex_.emplace(at, static_cast<uint32_t>(clist_.size())).second) clist_.push_back(at);
                 }
@@ -1682,27 +1686,45 @@ class Gen {
                 flip_[t].clear();
                 break;
             case K_REAL: {
-                std::vector<std::string> m = coefs(o.coef, 4);
+                const bool unit = o.special == SP_UNIT;  // m00 = m11 = 1
+                std::vector<std::string> m = unit ? coefs(o.coef + 1, 2) : coefs(o.coef, 4);
+                if (unit) m = {std::string(), m[0], m[1], std::string()};
                 if (!flip_[t].empty()) {  // X U X = [[m3, m2], [m1, m0]] where the thread's bit t is flipped
                     const std::string& p = flip_[t];
                     const std::vector<std::string> c = m;
-                    m = {sel(c[3], c[0], p), sel(c[2], c[1], p), sel(c[1], c[2], p), sel(c[0], c[3], p)};
+                    m[1] = sel(c[2], c[1], p);
+                    m[2] = sel(c[1], c[2], p);
+                    if (!unit) {
+                        m[0] = sel(c[3], c[0], p);
+                        m[3] = sel(c[0], c[3], p);
+                    }
                 }
                 for (int j : pairs(t, o.creg))
                     for (int s = 0; s < NS_; ++s) {
                         Cx a = A_[s][j], b = A_[s][j | (1 << t)];
-                        A_[s][j] = lin({{m[0], &a, 0}, {m[1], &b, 0}});
-                        A_[s][j | (1 << t)] = lin({{m[2], &a, 0}, {m[3], &b, 0}});
+                        if (unit) {
+                            A_[s][j] = lin({{m[1], &b, 0}}, &a);
+                            A_[s][j | (1 << t)] = lin({{m[2], &a, 0}}, &b);
+                        } else {
+                            A_[s][j] = lin({{m[0], &a, 0}, {m[1], &b, 0}});
+                            A_[s][j | (1 << t)] = lin({{m[2], &a, 0}, {m[3], &b, 0}});
+                        }
                     }
                 break;
             }
             case K_RX: {
-                const std::vector<std::string> m = coefs(o.coef, 2);
+                const bool unit = o.special == SP_UNIT;  // c = 1
+                const std::vector<std::string> m = unit ? coefs(o.coef + 1, 1) : coefs(o.coef, 2);
                 for (int j : pairs(t, o.creg))
                     for (int s = 0; s < NS_; ++s) {
                         Cx a = A_[s][j], b = A_[s][j | (1 << t)];
-                        A_[s][j] = lin({{m[0], &a, 0}, {m[1], &b, 3}});
-                        A_[s][j | (1 << t)] = lin({{m[0], &b, 0}, {m[1], &a, 3}});
+                        if (unit) {
+                            A_[s][j] = lin({{m[0], &b, 3}}, &a);
+                            A_[s][j | (1 << t)] = lin({{m[0], &a, 3}}, &b);
+                        } else {
+                            A_[s][j] = lin({{m[0], &a, 0}, {m[1], &b, 3}});
+                            A_[s][j | (1 << t)] = lin({{m[0], &b, 0}, {m[1], &a, 3}});
+                        }
                     }
                 break;
             }

@@ -1023,6 +1023,140 @@ void unnormalize_hadamards(std::vector<GOp>* gops) {
     }
 }
 
+void simplify_plain(std::vector<GOp>* gops) {
+    for (GOp& g : *gops) {
+        g.slot = -1;
+        g.bkind = 0;
+    }
+    fuse_single_qubit(gops);
+    unnormalize_hadamards(gops);
+}
+
+namespace {
+
+// Scalars taken out of a pass's gates (normalize_passes): at most
+// NORM_GROUP in a row before one gate takes their product back.  A gate is
+// left as it is where its scalar is below 2^-24 or the group has already
+// taken out 2^-64 (amplitudes grow by the inverse until the scalar is put
+// back, and float pairs need the range below them).  At random angles a
+// scalar is about 1/2 in the geometric mean and both limits are next to
+// never met (4e-8 per gate, below 1e-9 per group), so that passes which
+// differ only in their angles stay alike and share one compiled kernel.
+constexpr int NORM_GROUP = 16;
+constexpr double NORM_MIN = 0x1p-24, NORM_TOTAL = 0x1p-64;
+
+bool uncontrolled(const KOp& o) { return o.cthr == 0 && o.creg == 0; }
+
+// a rotation with equal diagonal entries, or a two-valued phase of register
+// bits: the scalar that makes its first diagonal entry 1
+bool scalar_of(const KOp& o, const double* c, cd* f) {
+    if (!uncontrolled(o)) return false;
+    if (o.kind == K_REAL) {
+        if (c[0] != c[3]) return false;
+        *f = cd(c[0], 0.0);
+    } else if (o.kind == K_RX) {
+        *f = cd(c[0], 0.0);
+    } else if (o.kind == K_DIAG) {
+        if (o.flags & (F_D0_ONE | F_D1_SPEC | F_UNIFORM | F_TPAR)) return false;
+        *f = cd(c[0], c[1]);
+    } else {
+        return false;
+    }
+    return std::abs(*f) >= NORM_MIN;
+}
+
+// number of (complex) coefficients a scalar multiplies into at no cost: the
+// op already applies general complex numbers to every amplitude
+int free_scalar_coefs(const KOp& o, bool probes) {
+    if (!uncontrolled(o)) return 0;
+    if (o.kind == K_DENSE) return 4;
+    if (o.kind == K_DENSE2) return 16;
+    // a phase of thread bits joins the round's phase, which multiplies every
+    // amplitude (at the round's end: too late for probes of the same round)
+    if (!probes && o.kind == K_DIAG && (o.flags & F_UNIFORM) && (o.flags & F_TPAR) && !(o.flags & (F_D0_ONE | F_D1_SPEC))) return 2;
+    return 0;
+}
+
+void scale_complex(double* c, int n, cd z) {
+    for (int i = 0; i < n; ++i) {
+        const cd v = cd(c[2 * i], c[2 * i + 1]) * z;
+        c[2 * i] = v.real();
+        c[2 * i + 1] = v.imag();
+    }
+}
+
+}  // namespace
+
+void normalize_passes(HostPlan* plan) {
+    if (!plan->binds.empty()) return;
+    for (const PassDesc& pd : plan->passes) {
+        if (pd.type != PASS_TILE) continue;
+        std::vector<int> ops;  // in execution order
+        for (int si = pd.step_begin; si < pd.step_begin + pd.step_count; ++si)
+            for (int oi = 0; oi < plan->steps[si].op_count; ++oi) ops.push_back(plan->steps[si].op_begin + oi);
+        std::vector<double> z2(ops.size(), 1.0);  // factor on |state|^2 from this op on
+        for (size_t i0 = 0, i1 = 0; i0 < ops.size(); i0 = i1) {
+            // the group, and the op of it that takes the product of the scalars
+            // back: one that does so at no cost, else a phase that stays in
+            // its full form, else (the product is then real) a rotation
+            size_t keeper = ops.size(), last_diag = ops.size(), last_rot = ops.size();
+            int count = 0;
+            cd f;
+            for (i1 = i0; i1 < ops.size() && count <= NORM_GROUP; ++i1) {
+                const KOp& o = plan->ops[ops[i1]];
+                if (free_scalar_coefs(o, pd.nprobe > 0)) keeper = i1;
+                if (!scalar_of(o, plan->coef.data() + o.coef, &f)) continue;
+                (o.kind == K_DIAG ? last_diag : last_rot) = i1;
+                ++count;
+            }
+            if (keeper == ops.size()) keeper = last_diag < ops.size() ? last_diag : last_rot;
+            if (keeper == ops.size()) continue;
+            cd total(1.0, 0.0);
+            for (size_t i = i0; i < i1; ++i) {
+                KOp& o = plan->ops[ops[i]];
+                double* c = plan->coef.data() + o.coef;
+                if (i == keeper || !scalar_of(o, c, &f) || std::abs(total * f) < NORM_TOTAL) continue;
+                total *= f;
+                z2[i] /= std::norm(f);
+                if (o.kind == K_REAL) {
+                    c[1] /= c[0];
+                    c[2] /= c[0];
+                    c[0] = c[3] = 1.0;
+                    o.special = SP_UNIT;
+                } else if (o.kind == K_RX) {
+                    c[1] /= c[0];
+                    c[0] = 1.0;
+                    o.special = SP_UNIT;
+                } else {
+                    const cd d1 = cd(c[2], c[3]) / f;
+                    c[0] = 1.0;
+                    c[1] = 0.0;
+                    c[2] = d1.real();
+                    c[3] = d1.imag();
+                    o.flags |= F_D0_ONE;
+                }
+            }
+            if (total == cd(1.0, 0.0)) continue;
+            const KOp& o = plan->ops[ops[keeper]];
+            double* c = plan->coef.data() + o.coef;
+            if (o.kind == K_REAL || o.kind == K_RX) {
+                for (int i = 0; i < (o.kind == K_REAL ? 4 : 2); ++i) c[i] *= total.real();
+            } else {
+                scale_complex(c, o.kind == K_DIAG ? 2 : free_scalar_coefs(o, false), total);
+            }
+            z2[keeper] *= std::norm(total);
+        }
+        // reverse sweeps: both states carry the scalars taken out so far, so a
+        // probe's sum carries their squared magnitude
+        double z = 1.0;
+        for (size_t i = 0; i < ops.size() && pd.nprobe > 0; ++i) {
+            const KOp& o = plan->ops[ops[i]];
+            if (o.kind == K_PROBE) plan->coef[o.coef] /= z;
+            z *= z2[i];
+        }
+    }
+}
+
 namespace {
 
 // bits of the register index an op of a round acts on non-diagonally

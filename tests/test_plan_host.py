@@ -336,3 +336,71 @@ def test_edge_sizes(precision):
         with pytest.raises(nat.QfvmError) as err:
             helpers.host_plan(n, [workloads.named("h", (0,))], precision)
         assert "qubit count out of range" in str(err.value)
+
+
+@pytest.mark.parametrize("precision,T,R", [(0, 11, 4), (2, 12, 3), (1, 13, 5)])
+@pytest.mark.parametrize("gates", ["rot", "mixed", "one", "dense"])
+@pytest.mark.parametrize("angle", [None, 0.0, np.pi / 2, np.pi, np.pi - 1e-5, -np.pi])
+def test_normalized_passes(precision, T, R, gates, angle):
+    """Scalars taken out of a pass's rotations and phases go back into one of
+    its gates: same state, at random angles and where a rotation's diagonal
+    vanishes (left as it is) or nearly does (|c| = 5e-6: unit form with
+    off-diagonal entries of 2e5).  At most about 8 gates deep on any
+    amplitude's path per layer and 4 layers: rounding stays below 1e-13."""
+    from pyquafu_gb300 import ir
+
+    n = T + 2
+    rng = np.random.default_rng(T + R)
+    ops = []
+
+    def rot(name, q):
+        th = float(rng.uniform(0, 2 * np.pi)) if angle is None else angle
+        ops.append(ir.Op(name, ir.NAMED_KIND[name], (q,), 0, (th,)))
+
+    for layer in range(1 if gates == "one" else 4):
+        if gates == "one":
+            rot("ry", n - 1)
+            continue
+        for q in range(n):
+            rot(["ry", "rx"][(q + layer) % 2] if gates != "mixed" else ["ry", "rz", "rx"][(q + layer) % 3], q)
+        if gates == "dense":
+            z, _ = np.linalg.qr(rng.normal(size=(2, 2)) + 1j * rng.normal(size=(2, 2)))
+            ops.append(workloads.matrix_gate("u", (layer,), z))
+            z, _ = np.linalg.qr(rng.normal(size=(4, 4)) + 1j * rng.normal(size=(4, 4)))
+            ops.append(workloads.matrix_gate("u2", (layer, n - 2), z))
+        ops += [workloads.named("cx", (q, q + 1), ncontrols=1) for q in range(n - 1)]
+    plan = helpers.host_plan(n, ops, precision, T, R)
+    psi = helpers.random_state(n, 5)
+    ref = oracle.simulate(n, ops, psi.copy())
+    assert np.abs(helpers.interpret(plan, psi) - ref).max() < 1e-13
+    unit = [int(o["special"]) for o in plan["ops"] if int(o["kind"]) in (helpers.K_REAL, helpers.K_RX)]
+    full = angle is not None and abs(angle) == np.pi  # |cos| = 6e-17
+    assert (sum(unit) == 0) == (full or gates == "one")
+
+
+@pytest.mark.parametrize("n,precision", [(13, 0), (14, 1), (13, 2)])
+def test_normalized_sweep_probes(n, precision):
+    """A reverse sweep planned at given angles takes scalars out of its
+    passes; its probes are rescaled (gradients against the oracle, angles
+    near pi among them)."""
+    ops, _ = workloads.hea(n, 2, seed=n)
+    for o in ops[::7]:
+        if o.slot >= 0:
+            o.params = (np.pi - 1e-4 * (1 + o.slot),)
+    plan = helpers.host_plan(n, ops, precision, adjoint=True)
+    assert len(plan["binds"]) == 0
+    # a round applies its thread-bit phases at its end, after its probes: such
+    # a phase must not carry the scalars of a pass with probes
+    for o in plan["ops"]:
+        if int(o["kind"]) == helpers.K_DIAG and int(o["flags"]) & 4 and not int(o["flags"]) & 1:
+            d = plan["coef"][int(o["coef"]): int(o["coef"]) + 2]
+            assert abs(np.hypot(*d) - 1) < 1e-15
+    assert any(int(o["special"]) == 1 for o in plan["ops"] if int(o["kind"]) == helpers.K_REAL)
+    terms = workloads.zz_x_hamiltonian(n, seed=n)
+    psi = oracle.simulate(n, ops)
+    vals = helpers.interpret2(plan, psi, oracle.apply_hamiltonian(psi, terms))
+    got = np.zeros(max(o.slot for o in ops) + 1)
+    for v, s in zip(vals, plan["probe_slots"]):
+        got[s] += v
+    ref = oracle.grad_adjoint(n, ops, [o.slot for o in ops], terms)
+    np.testing.assert_allclose(got, ref, atol=1e-11)
