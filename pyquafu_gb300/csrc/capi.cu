@@ -370,47 +370,20 @@ int sv_sample(qfvm_sv* sv, const double* uni, int64_t shots, uint64_t* out) {
     if (shots < 0) return fail(QFVM_ERR_INVALID, "negative shot count");
     if (shots == 0) return QFVM_OK;
     if (!uni || !out) return fail(QFVM_ERR_INVALID, "null sample buffer");
-    // the approximate total (parallel FP64 block sums) fixes the candidate binades
-    const uint64_t bs = std::min<uint64_t>(4096, sv->N);
-    const uint64_t nbs = sv->N / bs;
-    const uint64_t nb = (sv->N + SAMPLE_BS - 1) / SAMPLE_BS;
-    const size_t b_bsum = align256(nbs * 8), b_pre = align256((nbs + 1) * 8);
-    const size_t b_cnt = align256(static_cast<size_t>(SAMPLE_BINADES) * nb * 8);
-    const size_t b_ties = align256(static_cast<size_t>(SAMPLE_BINADES) * nb);
-    const size_t b_start = align256((nb + 1) * 8);
-    QSV_TRY(sv->sample_blk.ensure(b_bsum + b_pre + b_cnt + b_ties + b_start + 256));
-    char* blk = static_cast<char*>(sv->sample_blk.p);
-    double* dbsum = reinterpret_cast<double*>(blk);
-    double* dpre = reinterpret_cast<double*>(blk + b_bsum);
-    uint64_t* dcnt = reinterpret_cast<uint64_t*>(blk + b_bsum + b_pre);
-    uint8_t* dties = reinterpret_cast<uint8_t*>(blk + b_bsum + b_pre + b_cnt);
-    double* dstart = reinterpret_cast<double*>(blk + b_bsum + b_pre + b_cnt + b_ties);
-    int64_t* dseq = reinterpret_cast<int64_t*>(blk + b_bsum + b_pre + b_cnt + b_ties + b_start);
+    QSV_TRY(sv->sample_blk.ensure(sample_scratch_bytes(sv->N)));
+    SampleScratch w;
+    sample_scratch(sv->N, sv->sample_blk.p, &w);
     const size_t sz = static_cast<size_t>(shots);
     QSV_TRY(sv->sample_shots.ensure(align256(sz * 8) * 2));
     char* sb = static_cast<char*>(sv->sample_shots.p);
     double* duni = reinterpret_cast<double*>(sb);
     uint64_t* didx = reinterpret_cast<uint64_t*>(sb + align256(sz * 8));
     QSV_CUDA(cudaMemcpyAsync(duni, uni, sz * 8, cudaMemcpyHostToDevice, sv->stream), "uniform upload");
-    QSV_CUDA(launch_block_prefix(sv->precision, sv->d, sv->N, bs, dbsum, dpre, sv->stream), "block sums");
-    double total = 0.0;
-    QSV_CUDA(cudaMemcpyAsync(&total, dpre + nbs, 8, cudaMemcpyDeviceToHost, sv->stream), "total download");
-    QSV_CUDA(cudaStreamSynchronize(sv->stream), "sampling sync");
-    // binade of a value a little above the total (so a sequential total just
-    // past a power of two is still covered)
-    int e_top = 0;
-    const double tb = total * (1.0 + 1.0 / (1 << 20));
-    if (tb > 0.0 && std::isfinite(tb)) {
-        std::frexp(tb, &e_top);  // tb = f * 2^e_top, f in [0.5, 1)
-        e_top -= 1;
-    }
-    QSV_CUDA(launch_sample_binade(sv->precision, sv->d, sv->N, e_top, dcnt, dties, dstart, dseq, duni, shots, didx,
-                                  sv->stream),
-             "exact sampling");
+    QSV_CUDA(launch_sample(sv->precision, sv->d, sv->N, w, duni, shots, didx, sv->stream), "exact sampling");
     g_launches.fetch_add(5, std::memory_order_relaxed);
     int64_t seq = 0;
     QSV_CUDA(cudaMemcpyAsync(out, didx, sz * 8, cudaMemcpyDeviceToHost, sv->stream), "sample download");
-    QSV_CUDA(cudaMemcpyAsync(&seq, dseq, 8, cudaMemcpyDeviceToHost, sv->stream), "sample download");
+    QSV_CUDA(cudaMemcpyAsync(&seq, w.seq, 8, cudaMemcpyDeviceToHost, sv->stream), "sample download");
     QSV_CUDA(cudaStreamSynchronize(sv->stream), "sampling sync");
     sv->last_seq_blocks = seq;
     return check_status(sv->stream);

@@ -1,7 +1,6 @@
 // GB300 statevector kernels: whole-state passes, the generic k-target gate,
-// FP64 reductions (Pauli expectation, norms) and the sampling pipeline (block
-// sums, block prefix, per-shot locate, exact fallback).  The fused tile-pass
-// kernel is instantiated per precision in pass_c128.cu / pass_c64.cu.
+// FP64 reductions (Pauli expectation, norms).  The fused tile-pass kernel is
+// instantiated per precision in pass_c128.cu / pass_c64.cu.
 #include <atomic>
 
 #include "device.cuh"
@@ -181,66 +180,6 @@ __global__ void k_c64_to_c128(const float2* __restrict__ in, double2* __restrict
 }
 
 // ---------------------------------------------------------------------------
-// Sampling.  q_i = fl(fl(re^2) + fl(im^2)) exactly as the sequential scan of
-// measure_samples (statevector.hpp:1392-1396) forms it.
-// ---------------------------------------------------------------------------
-template <class P>
-__device__ __forceinline__ double prob_of(const typename P::G g) {
-    const double re = P::gre(g), im = P::gim(g);
-    return __dadd_rn(__dmul_rn(re, re), __dmul_rn(im, im));
-}
-
-template <class P>
-__global__ void __launch_bounds__(256) k_block_sums(const typename P::G* __restrict__ state, uint64_t bs,
-                                                    double* __restrict__ bsum) {
-    __shared__ double red[8];
-    const uint64_t b0 = static_cast<uint64_t>(blockIdx.x) * bs;
-    double s = 0.0;
-    for (uint64_t i = threadIdx.x; i < bs; i += 256) s += prob_of<P>(state[b0 + i]);
-    s = block_sum<256>(s, red);
-    if (threadIdx.x == 0) bsum[blockIdx.x] = s;
-}
-
-// Exclusive prefix over nb block sums (one CTA of 1024 threads); pre[nb] = total.
-__global__ void __launch_bounds__(1024) k_scan_blocks(const double* __restrict__ bsum, uint64_t nb,
-                                                      double* __restrict__ pre) {
-    __shared__ double wsum[32];
-    __shared__ double carry_s;
-    if (threadIdx.x == 0) carry_s = 0.0;
-    __syncthreads();
-    const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (uint64_t base = 0; base < nb; base += 1024) {
-        const uint64_t i = base + threadIdx.x;
-        const double v = i < nb ? bsum[i] : 0.0;
-        double x = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double y = __shfl_up_sync(0xffffffffu, x, o);
-            if (l >= o) x += y;
-        }
-        if (l == 31) wsum[w] = x;
-        __syncthreads();
-        if (w == 0) {
-            double z = wsum[l];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const double y = __shfl_up_sync(0xffffffffu, z, o);
-                if (l >= o) z += y;
-            }
-            wsum[l] = z;
-        }
-        __syncthreads();
-        const double carry = carry_s;
-        const double incl = x + (w > 0 ? wsum[w - 1] : 0.0) + carry;
-        if (i < nb) pre[i] = incl - v;
-        __syncthreads();
-        if (threadIdx.x == 1023) carry_s = incl;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) pre[nb] = carry_s;
-}
-
-// ---------------------------------------------------------------------------
 // Host launchers
 // ---------------------------------------------------------------------------
 // Shapes picked by the autotuner per (arithmetic, pass kind, qubit count),
@@ -394,19 +333,5 @@ cudaError_t launch_reduce_partials(const double* dpartial, int nblocks, int nter
     k_reduce_partials<<<1, 256, 0, st>>>(dpartial, nblocks, nterms, dout);
     return cudaGetLastError();
 }
-
-cudaError_t launch_block_prefix(int precision, const void* state, uint64_t N, uint64_t bs, double* dbsum,
-                                double* dpre, cudaStream_t st) {
-    const uint64_t nb = N / bs;
-    if (precision == QFVM_C64)
-        k_block_sums<P32><<<static_cast<unsigned>(nb), 256, 0, st>>>(static_cast<const float2*>(state), bs, dbsum);
-    else
-        k_block_sums<P64><<<static_cast<unsigned>(nb), 256, 0, st>>>(static_cast<const double2*>(state), bs, dbsum);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_scan_blocks<<<1, 1024, 0, st>>>(dbsum, nb, dpre);
-    return cudaGetLastError();
-}
-
 
 }  // namespace qsv

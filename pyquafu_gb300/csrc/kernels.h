@@ -48,19 +48,27 @@ cudaError_t launch_expect_x(int precision, const void* state, uint64_t N, uint64
                             const uint64_t* dzm, const int32_t* dny, int nterms, double* dpartial, int nblocks,
                             cudaStream_t st);
 cudaError_t launch_reduce_partials(const double* dpartial, int nblocks, int nterms, double* dout, cudaStream_t st);
-// Exact parallel sampling (sample.cu): blocks of SAMPLE_BS amplitudes, grid
-// counts for SAMPLE_BINADES binades below 2^e_top.  cnt: SAMPLE_BINADES * nb
-// uint64, ties: SAMPLE_BINADES * nb bytes, start: nb + 1 doubles (the exact
-// running sum at every block start), seq: blocks summed element by element.
+// Exact parallel sampling (sample.cu) in blocks of SAMPLE_BS amplitudes.
 constexpr int SAMPLE_BS = 4096;
-constexpr int SAMPLE_BINADES = 16;
-cudaError_t launch_sample_binade(int precision, const void* state, uint64_t N, int e_top, uint64_t* cnt,
-                                 uint8_t* ties, double* start, int64_t* seq, const double* uni, int64_t shots,
-                                 uint64_t* out, cudaStream_t st);
-// FP64 sums of |a|^2 over blocks of bs amplitudes and their exclusive prefix
-// (dpre[N / bs] = the parallel total)
-cudaError_t launch_block_prefix(int precision, const void* state, uint64_t N, uint64_t bs, double* dbsum,
-                                double* dpre, cudaStream_t st);
+constexpr int SAMPLE_SLOTS = 64;  // blocks whose inner running sums are kept for the shots
+struct SampleBlock {
+    uint64_t cnt[2];  // grid counts at binades e and (two) e + 1
+    int32_t e, two;
+};
+struct SampleScratch {
+    float* bsum;       // nb approximate block sums
+    double* pre;       // nb + 1: their exclusive prefix
+    SampleBlock* blk;  // nb
+    double* start;     // nb + 1: the exact running sum at every block start
+    int32_t* slot;     // nb
+    double* fine;      // SAMPLE_SLOTS * 1024 running sums
+    int64_t* seq;      // blocks resolved element by element
+};
+// Lays the scratch out from `base` (256-byte aligned) and returns its size.
+size_t sample_scratch(uint64_t N, void* base, SampleScratch* w);
+size_t sample_scratch_bytes(uint64_t N);
+cudaError_t launch_sample(int precision, const void* state, uint64_t N, const SampleScratch& w, const double* uni,
+                          int64_t shots, uint64_t* out, cudaStream_t st);
 
 }  // namespace qsv
 

@@ -242,3 +242,47 @@ def test_large_state_properties():
     assert abs(abs(psi0[0]) - 1.0) < 1e-11
     assert np.abs(psi0[1:]).max() < 1e-11
     assert abs(z - 1.0) < 1e-11
+
+
+def _sampling_states(n, kind):
+    rng = np.random.default_rng(31 * n + len(kind))
+    N = 1 << n
+    if kind == "decay":  # many binades within a block, and a long tail of amplitudes below the grid
+        return (2.0 ** -(np.arange(N) / 7.0 % 600)).astype(np.complex128)
+    if kind == "overflow":  # probabilities up to infinity
+        return (2.0 ** (np.arange(N) / 7.0 % 600)).astype(np.complex128)
+    if kind == "rise":  # the sum crosses a binade in almost every block
+        return np.exp(np.linspace(-40, 0, N)) * np.exp(1j * rng.uniform(0, 6, N))
+    if kind == "ties":  # |a|^2 = 2^-53 (1 + 2 k) around sums near 1: exact half-way cases throughout
+        a = np.full(N, 2.0 ** -26.5) * np.sqrt(1.0 + 2 * rng.integers(0, 4, N))
+        a[0] = 1.0
+        return a.astype(np.complex128)
+    if kind == "sparse":
+        a = np.zeros(N, dtype=np.complex128)
+        a[rng.choice(N, min(N, 5), replace=False)] = rng.normal(size=min(N, 5))
+        return a
+    if kind == "large":  # far from normalised
+        return helpers.random_state(n, n) * 2.0 ** 40
+    return np.full(N, 2.0 ** (-n / 2), dtype=np.complex128)  # uniform
+
+
+@pytest.mark.parametrize("kind", ["decay", "overflow", "rise", "ties", "sparse", "large", "uniform"])
+@pytest.mark.parametrize("n,precision", [(1, "c128"), (5, "c128"), (12, "c64"), (13, "c128"), (17, "c64"),
+                                         (19, "c128"), (23, "c128")])
+def test_sampling_structured_states(n, precision, kind):
+    """Index-exact sampling where the running sum meets its special cases:
+    binade crossings, exact ties, zeros, amplitudes below the grid, sums far
+    from one; shots at exact running sums and one ulp below."""
+    psi = _sampling_states(n, kind)
+    if precision == "c64":
+        with np.errstate(over="ignore", invalid="ignore"):
+            psi = psi.astype(np.complex64).astype(np.complex128)
+    cdf = oracle.sequential_cdf(psi)
+    rng = np.random.default_rng(n)
+    pick = cdf[rng.choice(cdf.size, min(cdf.size, 100), replace=False)]
+    u = np.concatenate([rng.random(500) * cdf[-1], [0.0, cdf[-1], np.nextafter(cdf[-1], 0.0)], pick,
+                        np.nextafter(pick, -1.0)])
+    st = engine.DeviceState(n, precision).upload(psi)
+    got = st.sample(u)
+    st.close()
+    assert np.array_equal(got, np.searchsorted(cdf, u, side="right"))  # the first index with u < cdf
