@@ -308,7 +308,7 @@ int sv_expect(qfvm_sv* sv, const uint64_t* xm, const uint64_t* zm, const int32_t
             groups[it - keys.begin()].push_back(t);
         }
     }
-    // launch batches of up to EXPECT_BATCH terms
+    // launch batches of terms of one flip mask
     std::vector<uint64_t> hz;
     std::vector<int32_t> hy;
     std::vector<std::pair<int64_t, int>> where;  // (term, batch slot)
@@ -319,9 +319,10 @@ int sv_expect(qfvm_sv* sv, const uint64_t* xm, const uint64_t* zm, const int32_t
     };
     std::vector<Batch> batches;
     for (size_t g = 0; g < groups.size(); ++g) {
-        for (size_t s = 0; s < groups[g].size(); s += EXPECT_BATCH) {
+        const size_t most = keys[g] == 0 ? EXPECT_Z_BATCH : EXPECT_BATCH;
+        for (size_t s = 0; s < groups[g].size(); s += most) {
             Batch b{keys[g], hz.size(), 0};
-            for (size_t k = s; k < groups[g].size() && k < s + EXPECT_BATCH; ++k) {
+            for (size_t k = s; k < groups[g].size() && k < s + most; ++k) {
                 hz.push_back(zm[groups[g][k]]);
                 hy.push_back(ny[groups[g][k]]);
                 ++b.count;
@@ -338,7 +339,7 @@ int sv_expect(qfvm_sv* sv, const uint64_t* xm, const uint64_t* zm, const int32_t
     uint64_t* dz = sv->masks.as<uint64_t>();
     int32_t* dy = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(sv->masks.p) + align256(nt * 8));
     double* dout = reinterpret_cast<double*>(reinterpret_cast<char*>(sv->masks.p) + align256(nt * 8) + align256(nt * 4));
-    QSV_TRY(sv->red.ensure(static_cast<size_t>(REDUCE_BLOCKS) * EXPECT_BATCH * sizeof(double)));
+    QSV_TRY(sv->red.ensure(static_cast<size_t>(REDUCE_BLOCKS) * EXPECT_Z_BATCH * sizeof(double)));
     QSV_CUDA(cudaMemcpyAsync(dz, hz.data(), nt * 8, cudaMemcpyHostToDevice, sv->stream), "term upload");
     QSV_CUDA(cudaMemcpyAsync(dy, hy.data(), nt * 4, cudaMemcpyHostToDevice, sv->stream), "term upload");
     const int nblocks = static_cast<int>(std::min<uint64_t>(REDUCE_BLOCKS, std::max<uint64_t>(1, sv->N / 2048)));
@@ -353,7 +354,8 @@ int sv_expect(qfvm_sv* sv, const uint64_t* xm, const uint64_t* zm, const int32_t
                                 sv->red.as<double>(), nblocks, sv->stream);
         }
         QSV_CUDA(e, "expectation");
-        QSV_CUDA(launch_reduce_partials(sv->red.as<double>(), nblocks, b.count, dout + b.first, sv->stream),
+        QSV_CUDA(launch_reduce_partials(sv->red.as<double>(), nblocks, b.x == 0 ? EXPECT_Z_BATCH : EXPECT_BATCH, b.count,
+                                        dout + b.first, sv->stream),
                  "expectation reduce");
         g_launches.fetch_add(2, std::memory_order_relaxed);
     }

@@ -311,9 +311,11 @@ cudaError_t launch_convert(bool to64, const void* in, void* out, uint64_t n, cud
 cudaError_t launch_expect_z(int precision, const void* state, uint64_t N, const uint64_t* dzm, int nterms,
                             double* dpartial, int nblocks, cudaStream_t st) {
     if (precision == QFVM_C64)
-        k_expect_z<P32><<<nblocks, 256, 0, st>>>(static_cast<const float2*>(state), N, dzm, nterms, dpartial);
+        k_expect_z<P32, EXPECT_Z_BATCH>
+            <<<nblocks, 256, 0, st>>>(static_cast<const float2*>(state), N, dzm, nterms, dpartial);
     else
-        k_expect_z<P64><<<nblocks, 256, 0, st>>>(static_cast<const double2*>(state), N, dzm, nterms, dpartial);
+        k_expect_z<P64, EXPECT_Z_BATCH>
+            <<<nblocks, 256, 0, st>>>(static_cast<const double2*>(state), N, dzm, nterms, dpartial);
     return cudaGetLastError();
 }
 
@@ -321,16 +323,17 @@ cudaError_t launch_expect_x(int precision, const void* state, uint64_t N, uint64
                             const uint64_t* dzm, const int32_t* dny, int nterms, double* dpartial, int nblocks,
                             cudaStream_t st) {
     if (precision == QFVM_C64)
-        k_expect_x<P32><<<nblocks, 256, 0, st>>>(static_cast<const float2*>(state), N, xmask, flip_q, dzm, dny,
-                                                 nterms, dpartial);
+        k_expect_x<P32, EXPECT_BATCH><<<nblocks, 256, 0, st>>>(static_cast<const float2*>(state), N, xmask, flip_q, dzm,
+                                                               dny, nterms, dpartial);
     else
-        k_expect_x<P64><<<nblocks, 256, 0, st>>>(static_cast<const double2*>(state), N, xmask, flip_q, dzm, dny,
-                                                 nterms, dpartial);
+        k_expect_x<P64, EXPECT_BATCH><<<nblocks, 256, 0, st>>>(static_cast<const double2*>(state), N, xmask, flip_q,
+                                                               dzm, dny, nterms, dpartial);
     return cudaGetLastError();
 }
 
-cudaError_t launch_reduce_partials(const double* dpartial, int nblocks, int nterms, double* dout, cudaStream_t st) {
-    k_reduce_partials<<<1, 256, 0, st>>>(dpartial, nblocks, nterms, dout);
+cudaError_t launch_reduce_partials(const double* dpartial, int nblocks, int stride, int nterms, double* dout,
+                                   cudaStream_t st) {
+    k_reduce_partials<<<nterms, 256, 0, st>>>(dpartial, nblocks, stride, dout);
     return cudaGetLastError();
 }
 

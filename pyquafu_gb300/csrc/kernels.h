@@ -7,7 +7,8 @@
 
 namespace qsv {
 
-constexpr int EXPECT_BATCH = 8;   // Pauli terms reduced per kernel launch
+constexpr int EXPECT_BATCH = 8;     // Pauli terms of one flip mask reduced per kernel launch
+constexpr int EXPECT_Z_BATCH = 16;  // Z-only terms (24 more would not fit the accumulators in 128 registers)
 constexpr int REDUCE_BLOCKS = 152 * 4;
 
 bool pass_shape_supported(int precision, int T, int R);
@@ -47,7 +48,8 @@ cudaError_t launch_expect_z(int precision, const void* state, uint64_t N, const 
 cudaError_t launch_expect_x(int precision, const void* state, uint64_t N, uint64_t xmask, int flip_q,
                             const uint64_t* dzm, const int32_t* dny, int nterms, double* dpartial, int nblocks,
                             cudaStream_t st);
-cudaError_t launch_reduce_partials(const double* dpartial, int nblocks, int nterms, double* dout, cudaStream_t st);
+cudaError_t launch_reduce_partials(const double* dpartial, int nblocks, int stride, int nterms, double* dout,
+                                   cudaStream_t st);
 // Exact parallel sampling (sample.cu) in blocks of SAMPLE_BS amplitudes.
 constexpr int SAMPLE_BS = 4096;
 constexpr int SAMPLE_SLOTS = 64;  // blocks whose inner running sums are kept for the shots

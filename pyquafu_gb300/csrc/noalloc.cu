@@ -168,22 +168,22 @@ extern "C" int qfvm_expect_device_noalloc(const void* dev_state, uint64_t state_
         while (i + cnt < m && cnt < EXPECT_BATCH && x_masks[order[i + cnt]] == x) ++cnt;
         if (x == 0) {
             if (precision == QFVM_C64)
-                k_expect_z<P32><<<nblocks, 256, 0, st>>>(static_cast<const float2*>(dev_state), state_len, d_zm + i,
+                k_expect_z<P32, EXPECT_BATCH><<<nblocks, 256, 0, st>>>(static_cast<const float2*>(dev_state), state_len, d_zm + i,
                                                          static_cast<int>(cnt), d_partial);
             else
-                k_expect_z<P64><<<nblocks, 256, 0, st>>>(static_cast<const double2*>(dev_state), state_len, d_zm + i,
+                k_expect_z<P64, EXPECT_BATCH><<<nblocks, 256, 0, st>>>(static_cast<const double2*>(dev_state), state_len, d_zm + i,
                                                          static_cast<int>(cnt), d_partial);
         } else {
             const int flip_q = 63 - __builtin_clzll(x);
             if (precision == QFVM_C64)
-                k_expect_x<P32><<<nblocks, 256, 0, st>>>(static_cast<const float2*>(dev_state), state_len, x, flip_q,
+                k_expect_x<P32, EXPECT_BATCH><<<nblocks, 256, 0, st>>>(static_cast<const float2*>(dev_state), state_len, x, flip_q,
                                                          d_zm + i, d_ny + i, static_cast<int>(cnt), d_partial);
             else
-                k_expect_x<P64><<<nblocks, 256, 0, st>>>(static_cast<const double2*>(dev_state), state_len, x, flip_q,
+                k_expect_x<P64, EXPECT_BATCH><<<nblocks, 256, 0, st>>>(static_cast<const double2*>(dev_state), state_len, x, flip_q,
                                                          d_zm + i, d_ny + i, static_cast<int>(cnt), d_partial);
         }
         NA_CUDA(cudaGetLastError(), "expectation kernel");
-        k_reduce_partials<<<1, 256, 0, st>>>(d_partial, nblocks, static_cast<int>(cnt), d_out + i);
+        k_reduce_partials<<<static_cast<unsigned>(cnt), 256, 0, st>>>(d_partial, nblocks, EXPECT_BATCH, d_out + i);
         NA_CUDA(cudaGetLastError(), "reduction kernel");
         i += cnt;
     }

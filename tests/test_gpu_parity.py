@@ -286,3 +286,42 @@ def test_sampling_structured_states(n, precision, kind):
     got = st.sample(u)
     st.close()
     assert np.array_equal(got, np.searchsorted(cdf, u, side="right"))  # the first index with u < cdf
+
+
+@pytest.mark.parametrize("n", [1, 2, 8, 9, 11, 12, 15])
+@pytest.mark.parametrize("precision", ["c128", "c64"])
+def test_expectation_term_groups(n, precision):
+    """Z-only terms below, at and above a shared batch (1, 3, 4, 16, 17 terms),
+    strings on every side of bits 8..10, groups of one and of several terms
+    that share a flip mask with even and odd numbers of Y; the same terms as
+    lam = H psi through the adjoint energy.  FP64 sums of at most 2^15 terms:
+    1e-13 (complex64 input is exact in FP64)."""
+    from pyquafu_gb300 import gradients
+
+    rng = np.random.default_rng(n)
+    psi = helpers.random_state(n, 7)
+    if precision == "c64":
+        psi = psi.astype(np.complex64).astype(np.complex128)
+    st = engine.DeviceState(n, precision).upload(psi)
+    letters = {0: "I", 1: "Z", 2: "X", 3: "Y"}
+    everyone = list(range(n))
+    for count in (1, 3, 4, 16, 17):
+        terms = [("".join(letters[int(v)] for v in rng.integers(0, 2, n)), everyone) for _ in range(count)]
+        got = st.expect(terms)
+        ref = [oracle.expect_pauli(psi, p, q) for p, q in terms]
+        np.testing.assert_allclose(got, ref, atol=1e-13, rtol=0)
+    flips = [("".join(letters[int(v)] for v in rng.integers(2, 4, n)), everyone) for _ in range(9)]  # one flip mask
+    singles = [("".join(letters[int(v)] for v in rng.integers(0, 4, n)), everyone) for _ in range(6)]
+    for terms in (flips, singles, flips[:1], [("Y", [n - 1])], [("X", [0])]):
+        got = st.expect(terms)
+        ref = [oracle.expect_pauli(psi, p, q) for p, q in terms]
+        np.testing.assert_allclose(got, ref, atol=1e-13, rtol=0)
+    st.close()
+    if precision == "c128" and n > 1:
+        ops, _ = workloads.hea(n, 1, seed=n)
+        h = [(float(rng.normal()), p, q) for p, q in flips + singles + [("Z" * n, everyone), ("Z", [n - 1])]]
+        h = [(c, p.replace("I", ""), [k for k, ch in zip(q, p) if ch != "I"]) for c, p, q in h]
+        e, g = gradients.adjoint(n, ops, h, "c128")
+        out = oracle.simulate(n, ops)
+        assert abs(e - sum(c * oracle.expect_pauli(out, p, q) for c, p, q in h)) < 1e-11
+        np.testing.assert_allclose(g, oracle.grad_adjoint(n, ops, [o.slot for o in ops], h), atol=1e-11)
