@@ -142,9 +142,12 @@ struct CifSpec {
     uint64_t condition;
 };
 int outcome_blocks_per_item(int n, int k);
-cudaError_t launch_measure(void* state, int n, const MeasureSpec& ms, int items, const double* duni, int draw,
-                           int ndraws, uint8_t* dcreg, int ncb, double* dpart, int32_t* doutcome, double* dscale,
-                           cudaStream_t st);
+// Measures or resets every item; the states of items c_begin .. items-1 are
+// collapsed (the outcomes alone matter for the others).  With `shared`, every
+// item's state is that one state and `state` receives the collapsed copies.
+cudaError_t launch_measure(const void* shared, void* state, int n, const MeasureSpec& ms, int items, int c_begin,
+                           const double* duni, int draw, int ndraws, uint8_t* dcreg, int ncb, double* dpart,
+                           int32_t* doutcome, double* dscale, cudaStream_t st);
 cudaError_t launch_cif_mask(const uint8_t* dcreg, int ncb, int items, const CifSpec& cs, uint8_t* dactive,
                             cudaStream_t st);
 cudaError_t launch_items_copy(void* state, int n, int items, const void* psi0, cudaStream_t st);

@@ -119,7 +119,7 @@ namespace qsv_capi {
 
 // Every pass of a plan over `items` states (shared coefficient pool).
 int run_plan_items(qfvm_plan* p, void* state, int items, const uint8_t* active, cudaStream_t st) {
-    p->chain_ok = false;  // inactive items keep their FP64 state: no float pairs between passes
+    if (active) p->chain_ok = false;  // inactive items keep their FP64 state: no float pairs between passes
     const HostPlan& hp = p->hp;
     for (size_t i = 0; i < hp.passes.size(); ++i) {
         const PassDesc& pd = hp.passes[i];
@@ -219,9 +219,18 @@ int qfvm_simulate_shots(int32_t num_qubits, int32_t num_cbits, const qfvm_op* op
     SHOT_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream");
     const size_t N = 1ULL << n;
     SHOT_TRY(dstate.ensure(static_cast<size_t>(chunk) * N * sizeof(double2)));
-    if (psi_in) {
-        SHOT_TRY(dpsi0.ensure(N * sizeof(double2)));
+    // Every shot starts from one state, and it stays one up to the first
+    // measure, reset or cif: that state is prepared once and copied to the shots.
+    SHOT_TRY(dpsi0.ensure(N * sizeof(double2)));
+    if (psi_in)
         SHOT_CUDA(cudaMemcpyAsync(dpsi0.p, psi_in, N * sizeof(double2), cudaMemcpyHostToDevice, st), "input upload");
+    else
+        SHOT_CUDA(launch_zero_items(QFVM_C128, dpsi0.p, n, 1, st), "initial state");
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    size_t first = 0;
+    if (!segs.empty() && segs[0].type == 0) {
+        SHOT_TRY(run_plan_items(segs[0].plan, dpsi0.p, 1, nullptr, st));
+        first = 1;
     }
     SHOT_TRY(duni.ensure(static_cast<size_t>(chunk) * std::max(ndraws, 1) * 8));
     SHOT_TRY(dcreg.ensure(static_cast<size_t>(chunk) * ncb));
@@ -242,17 +251,27 @@ int qfvm_simulate_shots(int32_t num_qubits, int32_t num_cbits, const qfvm_op* op
                                       cudaMemcpyHostToDevice, st),
                       "uniform upload");
         SHOT_CUDA(cudaMemsetAsync(dcreg.p, 0, static_cast<size_t>(items) * ncb, st), "classical bits");
-        if (psi_in) SHOT_CUDA(launch_items_copy(dstate.p, n, items, dpsi0.p, st), "initial states");
-        else SHOT_CUDA(launch_zero_items(QFVM_C128, dstate.p, n, items, st), "initial states");
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-        for (const auto& sg : segs) {
+        const bool last = c0 + items >= shots;
+        // a measure or reset of the shared state reads it from dpsi0 and writes
+        // the collapsed states; anything else starts from copies
+        bool shared = first < segs.size() && segs[first].type == 1;
+        if (!shared) {
+            SHOT_CUDA(launch_items_copy(dstate.p, n, items, dpsi0.p, st), "initial states");
+            g_launches.fetch_add(1, std::memory_order_relaxed);
+        }
+        for (size_t si = first; si < segs.size(); ++si) {
+            const Segment& sg = segs[si];
             if (sg.type == 0) {
                 SHOT_TRY(run_plan_items(sg.plan, dstate.p, items, nullptr, st));
             } else if (sg.type == 1) {
-                SHOT_CUDA(launch_measure(dstate.p, n, sg.ms, items, duni.as<double>(), sg.draw, ndraws,
-                                         dcreg.as<uint8_t>(), ncb, dpart, doutcome, dscale, st),
+                // nothing reads the other shots' states after the last operation
+                const int c_begin = si + 1 < segs.size() ? 0 : (last && final_state ? items - 1 : items);
+                SHOT_CUDA(launch_measure(shared ? dpsi0.p : nullptr, dstate.p, n, sg.ms, items, c_begin,
+                                         duni.as<double>(), sg.draw, ndraws, dcreg.as<uint8_t>(), ncb, dpart, doutcome,
+                                         dscale, st),
                           "measure");
                 g_launches.fetch_add(3, std::memory_order_relaxed);
+                shared = false;
             } else {
                 SHOT_CUDA(launch_cif_mask(dcreg.as<uint8_t>(), ncb, items, sg.cs, dactive, st), "cif");
                 g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -261,7 +280,6 @@ int qfvm_simulate_shots(int32_t num_qubits, int32_t num_cbits, const qfvm_op* op
         }
         SHOT_CUDA(cudaMemcpyAsync(hcreg.data(), dcreg.p, static_cast<size_t>(items) * ncb, cudaMemcpyDeviceToHost, st),
                   "classical bits download");
-        const bool last = c0 + items >= shots;
         if (last && final_state)
             SHOT_CUDA(cudaMemcpyAsync(final_state, dstate.as<double2>() + static_cast<size_t>(items - 1) * N,
                                       N * sizeof(double2), cudaMemcpyDeviceToHost, st),

@@ -78,3 +78,30 @@ def test_input_state_and_chunk_of_one():
     ref_out, ref_final = oracle.simulate_shots(n, ops, ncb, uni, psi_in=psi)
     assert out.tolist() == ref_out
     assert np.max(np.abs(final - ref_final)) < 1e-12
+
+
+@pytest.mark.parametrize("n", [3, 8, 9, 14])
+@pytest.mark.parametrize("start", ["measure", "reset", "cif", "gates"])
+@pytest.mark.parametrize("end", ["measure", "gates"])
+@pytest.mark.parametrize("shots", [1, 9])
+def test_shared_first_state_and_unread_last_states(n, start, end, shots):
+    """Shots share one state up to the first measure, reset or cif, and only the
+    last shot's state is read after the last measure; measured qubits below,
+    at and above the 256 amplitudes a block reads together."""
+    rng = np.random.default_rng(n + shots)
+    ncb = 5
+    pick = [int(q) for q in rng.permutation(n)]
+    first = {"measure": ir.Op("measure", ir.OP_MEASURE, qbits=[n - 1, 0], cbits=[0, 1]),
+             "reset": ir.Op("reset", ir.OP_RESET, qbits=[0, n - 1]),
+             "cif": ir.Op("cif", ir.OP_CIF, cbits=[0], condition=0, body=[named("x", (n - 1,))]),
+             "gates": named("h", (0,))}[start]
+    ops = [first] + workloads.random_layers(n, 2, seed=n)
+    ops.append(ir.Op("measure", ir.OP_MEASURE, qbits=pick[:3], cbits=[2, 0, 4]))
+    ops += workloads.random_layers(n, 1, seed=n + 1) if end == "gates" else []
+    psi = helpers.random_state(n, 3)
+    qfvm.set_seed(17)
+    out, final = qfvm._shots(n, ncb, ops, psi, shots)
+    uni = qfvm.last_uniforms.reshape(shots, draws(ops))
+    ref_out, ref_final = oracle.simulate_shots(n, ops, ncb, uni, psi)
+    assert out.tolist() == ref_out
+    assert np.max(np.abs(final - ref_final)) < 1e-12
