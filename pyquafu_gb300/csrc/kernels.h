@@ -159,9 +159,14 @@ constexpr int MAX_CHANNEL_OPS = 8;
 int channel_blocks_per_item(int n);  // CTAs per item of the Kraus-norm reduction
 // cross: some Kraus operator's Gram matrix K^dagger K has a nonzero
 // off-diagonal entry (the norms then need sum conj(a) c as well)
+// One channel on every item.  A Kraus channel leaves the item's state
+// unnormalised by 1 / dscale[item] where that factor is moderate.
 cudaError_t launch_channel(void* state, int n, int q, int m, int kraus, int cross, const double* dmats,
                            const double* dprobs, int items, const double* duni, int draw, int ndraws, double* dpart,
-                           double* dimat, cudaStream_t st);
-cudaError_t launch_item_sample(const void* state, int n, int items, const double* duni, int draw, int ndraws,
-                               uint64_t* dout, cudaStream_t st);
+                           double* dimat, double* dscale, cudaStream_t st);
+cudaError_t launch_fill_ones(double* d, int count, cudaStream_t st);
+// values[item * per + t] *= scale[item]^2
+cudaError_t launch_scale_items(double* values, int items, int per, const double* dscale, cudaStream_t st);
+cudaError_t launch_item_sample(const void* state, int n, int items, const double* dscale, const double* duni, int draw,
+                               int ndraws, uint64_t* dout, cudaStream_t st);
 }  // namespace qsv

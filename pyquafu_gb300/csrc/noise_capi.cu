@@ -139,7 +139,7 @@ int qfvm_simulate_noise(int32_t num_qubits, const qfvm_op* ops, int64_t n_ops, c
     const uint64_t epi = N / chunk_amps;  // expectation chunks per item
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
-    const size_t per_item = (sizeof(double2) << n) + 8u * ndraws + 8u * bpi * (MAX_CHANNEL_OPS + 1) + 64 + 8 +
+    const size_t per_item = (sizeof(double2) << n) + 8u * ndraws + 8u * bpi * (MAX_CHANNEL_OPS + 1) + 64 + 16 +
                             8u * static_cast<size_t>(n_terms) * (epi + 1);
     int64_t chunk = static_cast<int64_t>((free_b / 2) / per_item);
     if (chunk < 1) chunk = 1;
@@ -175,9 +175,17 @@ int qfvm_simulate_noise(int32_t num_qubits, const qfvm_op* ops, int64_t n_ops, c
     } while (0)
     NZ_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream");
     NZ_TRY(dstate.ensure(static_cast<size_t>(chunk) * N * sizeof(double2)));
-    if (psi_in) {
-        NZ_TRY(dpsi0.ensure(N * sizeof(double2)));
+    // the shots share one state up to the first channel: prepared once, then copied
+    NZ_TRY(dpsi0.ensure(N * sizeof(double2)));
+    if (psi_in)
         NZ_CUDA(cudaMemcpyAsync(dpsi0.p, psi_in, N * sizeof(double2), cudaMemcpyHostToDevice, st), "input upload");
+    else
+        NZ_CUDA(launch_zero_items(QFVM_C128, dpsi0.p, n, 1, st), "initial state");
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    size_t first = 0;
+    if (!segs.empty() && segs[0].type == 0) {
+        NZ_TRY(run_plan_items(segs[0].plan, dpsi0.p, 1, nullptr, st));
+        first = 1;
     }
     NZ_TRY(duni.ensure(static_cast<size_t>(chunk) * ndraws * 8));
     // scratch: channel data, channel norms, per-item matrices, samples, expectation chunks and values
@@ -187,7 +195,8 @@ int qfvm_simulate_noise(int32_t num_qubits, const qfvm_op* ops, int64_t n_ops, c
     const size_t b_smp = align256(static_cast<size_t>(chunk) * 8);
     const size_t b_ep = align256(static_cast<size_t>(chunk) * epi * std::max<int64_t>(n_terms, 1) * 8);
     const size_t b_ev = align256(static_cast<size_t>(chunk) * std::max<int64_t>(n_terms, 1) * 8);
-    NZ_TRY(dscratch.ensure(b_cd + b_part + b_imat + b_smp + b_ep + b_ev));
+    const size_t b_sc = align256(static_cast<size_t>(chunk) * 8);
+    NZ_TRY(dscratch.ensure(b_cd + b_part + b_imat + b_smp + b_ep + b_ev + b_sc));
     char* sp = static_cast<char*>(dscratch.p);
     double* dcd = reinterpret_cast<double*>(sp);
     double* dpart = reinterpret_cast<double*>(sp + b_cd);
@@ -195,6 +204,7 @@ int qfvm_simulate_noise(int32_t num_qubits, const qfvm_op* ops, int64_t n_ops, c
     uint64_t* dsmp = reinterpret_cast<uint64_t*>(sp + b_cd + b_part + b_imat);
     double* depart = reinterpret_cast<double*>(sp + b_cd + b_part + b_imat + b_smp);
     double* dev = reinterpret_cast<double*>(sp + b_cd + b_part + b_imat + b_smp + b_ep);
+    double* dscale = reinterpret_cast<double*>(sp + b_cd + b_part + b_imat + b_smp + b_ep + b_ev);
     if (!cdata.empty())
         NZ_CUDA(cudaMemcpyAsync(dcd, cdata.data(), cdata.size() * 8, cudaMemcpyHostToDevice, st), "channel upload");
     uint64_t* dx = nullptr;
@@ -228,21 +238,22 @@ int qfvm_simulate_noise(int32_t num_qubits, const qfvm_op* ops, int64_t n_ops, c
         NZ_CUDA(cudaMemcpyAsync(duni.p, uniforms + c0 * ndraws, static_cast<size_t>(items) * ndraws * 8,
                                 cudaMemcpyHostToDevice, st),
                 "uniform upload");
-        if (psi_in) NZ_CUDA(launch_items_copy(dstate.p, n, items, dpsi0.p, st), "initial states");
-        else NZ_CUDA(launch_zero_items(QFVM_C128, dstate.p, n, items, st), "initial states");
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-        for (const auto& sg : segs) {
+        NZ_CUDA(launch_items_copy(dstate.p, n, items, dpsi0.p, st), "initial states");
+        NZ_CUDA(launch_fill_ones(dscale, items, st), "initial scales");
+        g_launches.fetch_add(2, std::memory_order_relaxed);
+        for (size_t si = first; si < segs.size(); ++si) {
+            const NoiseSegment& sg = segs[si];
             if (sg.type == 0) {
                 NZ_TRY(run_plan_items(sg.plan, dstate.p, items, nullptr, st));
             } else {
                 NZ_CUDA(launch_channel(dstate.p, n, sg.q, sg.m, sg.kraus, sg.cross, dcd + sg.mat_off, dcd + sg.prob_off,
                                        items,
-                                       duni.as<double>(), sg.draw, ndraws, dpart, dimat, st),
+                                       duni.as<double>(), sg.draw, ndraws, dpart, dimat, dscale, st),
                         "channel");
                 g_launches.fetch_add(sg.kraus ? 3 : 2, std::memory_order_relaxed);
             }
         }
-        NZ_CUDA(launch_item_sample(dstate.p, n, items, duni.as<double>(), ndraws - 1, ndraws, dsmp, st), "sample");
+        NZ_CUDA(launch_item_sample(dstate.p, n, items, dscale, duni.as<double>(), ndraws - 1, ndraws, dsmp, st), "sample");
         g_launches.fetch_add(1, std::memory_order_relaxed);
         NZ_CUDA(cudaMemcpyAsync(samples + c0, dsmp, static_cast<size_t>(items) * 8, cudaMemcpyDeviceToHost, st),
                 "sample download");
@@ -250,7 +261,8 @@ int qfvm_simulate_noise(int32_t num_qubits, const qfvm_op* ops, int64_t n_ops, c
             NZ_CUDA(launch_expect_seg(QFVM_C128, dstate.p, n, items, dx, dz, dy, dc, doptr, static_cast<int>(n_terms),
                                       depart, dev, st),
                     "expectation");
-            g_launches.fetch_add(2, std::memory_order_relaxed);
+            NZ_CUDA(launch_scale_items(dev, items, static_cast<int>(n_terms), dscale, st), "expectation scales");
+            g_launches.fetch_add(3, std::memory_order_relaxed);
             NZ_CUDA(cudaMemcpyAsync(expvals + c0 * n_terms, dev, static_cast<size_t>(items) * n_terms * 8,
                                     cudaMemcpyDeviceToHost, st),
                     "expectation download");

@@ -137,3 +137,31 @@ def test_dropin_simulator_on_protocol_objects():
         counts[st] = counts.get(st, 0) + 1
     assert res["counts"] == counts
     np.testing.assert_allclose(res["pauli_expects"], ref_e.mean(axis=0), atol=1e-12)
+
+
+@pytest.mark.parametrize("n,shots", [(2, 3), (9, 1), (13, 130)])
+@pytest.mark.parametrize("factor", [1.0, 2.0 ** -7, 2.0 ** 13, 3e-9])
+def test_kraus_norms_left_out_of_the_state(n, shots, factor):
+    """Kraus operators whose norms leave the state unnormalised by a moderate
+    factor, or one that has to be applied at once; their diagonal, off-diagonal,
+    zero-row and general forms; a channel first and last, and shots enough for
+    the long norm blocks (130 x 2^12 pairs)."""
+    rng = np.random.default_rng(n)
+    forms = [np.diag([1.0, 0.8]), np.diag([0.6, 1.0]), np.array([[0, 0.7], [0, 0]]), np.array([[0, 0.9], [0.5, 0]]),
+             rng.normal(size=(2, 2)) + 1j * rng.normal(size=(2, 2)), np.diag([0.5, 0.5j])]
+    ops = []
+    for layer in range(3):
+        for i, k in enumerate(forms):
+            ops.append(ir.channel_op(ir.OP_KRAUS, (layer + i) % n, [factor * k]))
+        ops += workloads.random_layers(n, 1, seed=layer)
+    ops.append(ir.channel_op(ir.OP_KRAUS, n - 1, [factor * np.diag([1.0, 0.3]), np.eye(2)]))
+    uni = np.zeros((shots, ir.noise_draws(ops)))  # always the first operator
+    uni[:, -1] = rng.random(shots)
+    psi = helpers.random_state(n, 6)
+    terms = [(1.0, "Z", [0]), (0.5, "XY", [0, n - 1])]
+    samples, expv = noise.simulate_noise(n, ops, shots, psi=psi, terms=terms, uniforms=uni)
+    k = min(shots, 3)
+    ref_s, ref_e = oracle.simulate_noise(n, ops, uni[:k], psi_in=psi, terms=terms)
+    assert samples.tolist()[:k] == ref_s
+    np.testing.assert_allclose(expv[:k], ref_e, atol=1e-12)
+    np.testing.assert_allclose(expv, np.broadcast_to(ref_e[:1], expv.shape), atol=1e-12)
