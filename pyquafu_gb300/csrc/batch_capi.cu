@@ -40,6 +40,8 @@ struct BatchGroup {
     int32_t* doptr = nullptr;   // observable o = terms [doptr[o], doptr[o + 1])
     int32_t* dtobs = nullptr;   // observable of every term
     double* epart = nullptr;    // per-chunk expectation sums
+    double* npart = nullptr;    // complex64: per-chunk |psi|^2 sums and 1 / <psi|psi> per item, else null
+    double* inv = nullptr;
     double* pvals = nullptr;    // items x nprobe probe values
     double* partial = nullptr;  // MAX_PASS_PROBES rows of per-tile probe sums
     int32_t* sptr = nullptr;    // slot -> probes (CSR)
@@ -263,10 +265,18 @@ int add_group(qfvm_batch* b, int n, const qfvm_op* ops, int64_t n_ops, const dou
         b_csr = align256(csr.size() * 4);
     }
     const size_t b_ep = align256(static_cast<size_t>(chunks) * n_obs * 8);
-    rc = g->scratch.ensure(b_ep + b_pv + b_part + b_csr);
+    // complex64 states drift from unit norm with the rounding of their gates'
+    // coefficients (about 3e-7 over 400 gates): their results are divided by <psi|psi>
+    const size_t b_np = storage == QFVM_C64 ? align256(static_cast<size_t>(chunks) * 8) : 0;
+    const size_t b_inv = storage == QFVM_C64 ? align256(static_cast<size_t>(n_items) * 8) : 0;
+    rc = g->scratch.ensure(b_ep + b_pv + b_part + b_csr + b_np + b_inv);
     if (rc != QFVM_OK) return bail(rc);
     char* sb = static_cast<char*>(g->scratch.p);
     g->epart = reinterpret_cast<double*>(sb);
+    if (storage == QFVM_C64) {
+        g->npart = reinterpret_cast<double*>(sb + b_ep + b_pv + b_part + b_csr);
+        g->inv = reinterpret_cast<double*>(sb + b_ep + b_pv + b_part + b_csr + b_np);
+    }
     if (grads) {
         g->pvals = reinterpret_cast<double*>(sb + b_ep);
         g->partial = reinterpret_cast<double*>(sb + b_ep + b_pv);
@@ -345,7 +355,7 @@ int enqueue_group(qfvm_batch* b, BatchGroup* g, int mode, uint64_t* nk) {
                        "batched global op");
     }
     QSV_LAUNCH(launch_expect_seg(storage, g->psi.p, n, items, g->dx, g->dz, g->dy, g->dc, g->doptr, g->nobs, g->epart,
-                                 expv, st),
+                                 expv, g->npart, g->inv, st),
                "batched expectation");
     ++*nk;  // the segmented sum
     if (mode == 0) return QFVM_OK;
@@ -389,7 +399,7 @@ int enqueue_group(qfvm_batch* b, BatchGroup* g, int mode, uint64_t* nk) {
         }
     }
     if (g->nslots)
-        QSV_LAUNCH(launch_slot_gather(g->pvals, g->nprobe, items, g->sptr, g->sidx, g->nslots, grads, st),
+        QSV_LAUNCH(launch_slot_gather(g->pvals, g->nprobe, items, g->sptr, g->sidx, g->nslots, g->inv, grads, st),
                    "slot sums");
     return QFVM_OK;
 }

@@ -115,16 +115,18 @@ cudaError_t launch_bind(int arith, void* pool, uint64_t cstride, const Bind* dbi
 cudaError_t launch_replicate(int arith, void* pool, uint64_t cstride, uint64_t len, int items, cudaStream_t st);
 cudaError_t launch_zero_items(int storage, void* state, int n, int items, cudaStream_t st);
 uint64_t hamiltonian_chunk(int n);
+// Expectation values per item; npart / inv (complex64; null: as they are):
+// divided by the item's <psi|psi>, inv[item] = 1 / <psi|psi>.
 cudaError_t launch_expect_seg(int storage, const void* psi, int n, int items, const uint64_t* dx, const uint64_t* dz,
                               const int32_t* dny, const double* dc, const int32_t* doptr, int nobs, double* epart,
-                              double* out, cudaStream_t st);
+                              double* out, double* npart, double* inv, cudaStream_t st);
 cudaError_t launch_lambda_seg(int storage, const void* psi, void* lam, int n, int items, const uint64_t* dx,
                               const uint64_t* dz, const int32_t* dny, const double* dc, const int32_t* dtobs,
                               int nterms, int nobs, const double* dw, cudaStream_t st);
 cudaError_t launch_probe_reduce_seg(const double* partial, uint64_t ntiles, int tpi, int items, int np, double* out,
                                     int ostride, int ooff, cudaStream_t st);
 cudaError_t launch_slot_gather(const double* vals, int nprobe, int items, const int32_t* sptr, const int32_t* sidx,
-                               int nslots, double* grads, cudaStream_t st);
+                               int nslots, const double* inv, double* grads, cudaStream_t st);
 }  // namespace qsv
 
 namespace qsv {

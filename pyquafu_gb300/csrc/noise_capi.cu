@@ -259,7 +259,7 @@ int qfvm_simulate_noise(int32_t num_qubits, const qfvm_op* ops, int64_t n_ops, c
                 "sample download");
         if (n_terms > 0) {
             NZ_CUDA(launch_expect_seg(QFVM_C128, dstate.p, n, items, dx, dz, dy, dc, doptr, static_cast<int>(n_terms),
-                                      depart, dev, st),
+                                      depart, dev, nullptr, nullptr, st),
                     "expectation");
             NZ_CUDA(launch_scale_items(dev, items, static_cast<int>(n_terms), dscale, st), "expectation scales");
             g_launches.fetch_add(3, std::memory_order_relaxed);

@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 import oracle
-from pyquafu_gb300 import gradients, workloads
+from pyquafu_gb300 import gradients, ir, workloads
 from pyquafu_gb300.batch import BatchSession
 
 pytestmark = pytest.mark.gpu
@@ -130,3 +130,49 @@ def test_phase_gates_and_forward_only():
                 ev.append(oracle.energy(n, gradients.bind(ops, w), terms))
             fd[k] = (ev[0] - ev[1]) / (2 * h)
         np.testing.assert_allclose(g[0][i], fd, atol=1e-7)
+
+
+@pytest.mark.parametrize("n", [3, 8, 9, 11, 12, 14])
+@pytest.mark.parametrize("precision", ["c64", "c128"])
+def test_observable_forms(n, precision):
+    """Expectation values and lam = O psi of a group: one diagonal term, several,
+    one flipping term with an even and an odd number of Y (its coefficient a
+    float and not), and all of them, alone (no weights) and as weighted
+    observables of one group; RZ and RZZ bound without their global phase."""
+    rng = np.random.default_rng(n)
+    ops, _ = workloads.hea(n, 1, seed=n, encode=np.zeros(n))
+    nslots = max(o.slot for o in ops) + 1
+    ops.insert(n, ir.Op("rzz", ir.OP_RZZ, (0, n - 1), 0, (0.0,), slot=nslots))
+    nslots += 1
+    e = n - 1
+    observables = [[(1.0, "Z", [0])], [(0.5, "Z", [e]), (-0.25, "ZZ", [0, e]), (0.3, "ZZZ", [0, 1, e]), (1.0, "Z", [1])],
+                   [(0.5, "X", [e])], [(0.1, "Y", [0])], [(0.7, "XY", [0, e]), (0.2, "YX", [0, e]), (0.4, "ZX", [0, 1])]]
+    observables.append([t for o in observables for t in o])
+    items = 3
+    vals = rng.uniform(-np.pi, np.pi, (items, nslots))
+    vals[0, ::3] = np.pi
+    tol = 1e-5 if precision == "c64" else 1e-11
+    bound = [gradients.bind(ops, v) for v in vals]
+    states = [oracle.simulate(n, b) for b in bound]
+    ref_e = np.array([[sum(c * oracle.expect_pauli(s, p, q) for c, p, q in o) for o in observables] for s in states])
+    plain = [k for k, o in enumerate(ops) if o.name != "rzz"]  # the oracle's gradients know rx, ry, rz
+    weights = rng.normal(size=(items, len(observables)))
+
+    def ref_grad(i, terms):
+        g = oracle.grad_adjoint(n, bound[i], [o.slot if k in plain else -1 for k, o in enumerate(bound[i])], terms)
+        return np.append(g, np.zeros(nslots - len(g)))
+
+    mask = np.arange(nslots) != nslots - 1
+    with BatchSession(precision, grads=True) as bs:
+        bs.add_group(n, ops, observables, items, nslots)
+        ev, g = bs.run([vals], grads=True, weights=[weights])
+        np.testing.assert_allclose(ev[0], ref_e, atol=tol)
+        for i in range(items):
+            terms = [(c * weights[i, k], p, q) for k, o in enumerate(observables) for c, p, q in o]
+            np.testing.assert_allclose(g[0][i][mask], ref_grad(i, terms)[mask], atol=5 * tol)
+    for k, o in enumerate(observables):
+        with BatchSession(precision, grads=True) as bs:
+            bs.add_group(n, ops, o, items, nslots)
+            ev, g = bs.run([vals], grads=True)
+            np.testing.assert_allclose(ev[0][:, 0], ref_e[:, k], atol=tol)
+            np.testing.assert_allclose(g[0][1][mask], ref_grad(1, o)[mask], atol=tol)
