@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(256) k_bind(C* __restrict__ pool, uint64_t cst
         const Bind bd = binds[i - item * nb];
         const double th = static_cast<double>(bd.sign) * vals[item * nslots + bd.slot];
         double c[4];
-        const int m = bind_eval(bd.kind, th, c);
+        const int m = bind_eval(bd.unit ? QFVM_OP_P : bd.kind, th, c);
         C* dst = pool + item * cstride + bd.off;
         for (int k = 0; k < m; ++k) put_coef(dst + k, c[k]);
     }

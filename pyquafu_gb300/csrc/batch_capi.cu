@@ -170,7 +170,9 @@ int add_group(qfvm_batch* b, int n, const qfvm_op* ops, int64_t n_ops, const dou
     if (cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&g->done, cudaEventDisableTiming) != cudaSuccess)
         return bail(fail(QFVM_ERR_CUDA, "batch stream creation"));
-    int rc = make_plan_gops(n, arith, gops, b->T, b->R, &g->fwd);
+    int fT = b->T, fR = b->R;
+    if (fT <= 0 && fR <= 0) batch_forward_shape(arith, n, &fT, &fR);
+    int rc = make_plan_gops(n, arith, gops, fT, fR, &g->fwd);
     if (rc != QFVM_OK) return bail(rc);
     if (grads) {
         int aT = b->aT, aR = b->aR;

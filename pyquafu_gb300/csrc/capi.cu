@@ -670,6 +670,8 @@ int qfvm_plan_host_build_batched(int32_t num_qubits, int32_t precision, const qf
     if (adjoint) {
         if (!build_adjoint_sweep(gops, &sweep, &err)) return fail(QFVM_ERR_INVALID, err);
         resolve_shape(precision, 1, num_qubits, &T, &R);
+    } else {
+        batch_forward_shape(precision, num_qubits, &T, &R);
     }
     qfvm_plan* p = new qfvm_plan();
     if (!build_plan(num_qubits, store_precision(precision), adjoint ? sweep : gops, T, R, &p->hp, &err)) {

@@ -48,6 +48,11 @@ enum : uint8_t {
 enum : uint8_t { SP_NEG1 = 1, SP_I = 2, SP_NEGI = 3 };
 // K_REAL / K_RX `special`: both diagonal entries are exactly 1 (normalize_passes)
 enum : uint8_t { SP_UNIT = 1 };
+// K_DIAG `special` of a bound RZ / RZZ (unfix_bound): the device binds it as
+// diag(1, e^{i theta}), a global phase away.  A batch returns expectation
+// values and gradients, which that phase does not reach, and a phase with a
+// first entry of 1 touches half the amplitudes.
+enum : uint8_t { SP_BOUND_RZ = 4 };
 
 constexpr int MAXK = 6;  // largest dense target count held in a thread's registers (k_globalop, k_small)
 // Dense gates on MAXK+1 .. MAX_DENSE_TARGETS targets run one CTA per group of
@@ -89,7 +94,7 @@ struct Bind {
     uint32_t off;
     uint8_t kind;
     int8_t sign;
-    uint16_t pad;
+    uint16_t unit;  // 1: an RZ / RZZ bound without its global phase (SP_BOUND_RZ)
     int32_t slot;
 };
 static_assert(sizeof(Bind) == 12, "Bind layout");

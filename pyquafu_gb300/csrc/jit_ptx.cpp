@@ -1575,7 +1575,7 @@ class Gen {
                     const int h = (j >> t) & 1;
                     for (int s = 0; s < NS_; ++s) {
                         if (h == 0) {
-                            if (o.flags & F_D0_ONE) continue;
+                            if ((o.flags & F_D0_ONE) || o.special == SP_BOUND_RZ) continue;
                             A_[s][j] = phase(A_[s][j], {c[0], c[1]});
                         } else if (o.flags & F_D1_SPEC) {
                             A_[s][j] = special(A_[s][j], o.special);
@@ -1607,7 +1607,7 @@ class Gen {
             for (int j = 0; j < NA_; ++j) {
                 if ((static_cast<uint32_t>(j) & o.creg) != o.creg) continue;
                 const int par = __builtin_popcount(static_cast<uint32_t>(j) & o.preg) & 1;
-                if (par == 0 && !tpar && (o.flags & F_D0_ONE)) continue;
+                if (par == 0 && !tpar && ((o.flags & F_D0_ONE) || o.special == SP_BOUND_RZ)) continue;
                 for (int s = 0; s < NS_; ++s) A_[s][j] = phase(A_[s][j], f[par]);
             }
         }

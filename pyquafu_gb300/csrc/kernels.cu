@@ -200,6 +200,16 @@ void resolve_shape(int arith, int kind, int n, int* T, int* R) {
     else default_shape(n, arith, T, R);
 }
 
+void batch_forward_shape(int arith, int n, int* T, int* R) {
+    resolve_shape(arith, 0, n, T, R);
+    int dT = 0, dR = 0;
+    default_shape(n, arith, &dT, &dR);
+    if (arith == QFVM_C64 && *T == dT && *R == dR) {
+        *T = 12;
+        *R = 4;
+    }
+}
+
 bool set_tuned_shape(int arith, int kind, int n, int T, int R) {
     if (n < 0 || n > QFVM_MAX_QUBITS || (kind != 0 && kind != 1)) return false;
     const int a = (arith == QFVM_C64) ? 1 : (arith == QFVM_C128_DS ? 2 : 0);

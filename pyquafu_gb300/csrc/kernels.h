@@ -16,6 +16,11 @@ bool pass_shape_supported(int precision, int T, int R);
 // the autotuned one if set, else the built-in default.
 void resolve_shape(int arith, int kind, int n, int* T, int* R);
 bool set_tuned_shape(int arith, int kind, int n, int T, int R);
+// One-state shape of a batch group's forward plan (T = 0 asked for): as
+// resolve_shape, but complex64 groups default to (12, 4).  A hardware-efficient
+// ansatz puts most of its gates into the first pass, whose unrolled rounds at
+// five register qubits (22 K instructions) ran out of the instruction cache.
+void batch_forward_shape(int arith, int n, int* T, int* R);
 bool pass_shape_c128(int T, int R);
 bool pass_shape_c64(int T, int R);
 bool pass_shape_ds(int T, int R);

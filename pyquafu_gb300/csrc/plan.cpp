@@ -436,7 +436,7 @@ uint32_t push_coef(HostPlan* p, const GOp& g) {
     uint32_t off = static_cast<uint32_t>(p->coef.size());
     p->coef.insert(p->coef.end(), g.coef.begin(), g.coef.end());
     if (g.bkind != 0 && g.slot >= 0 && g.kind != K_PROBE)
-        p->binds.push_back(Bind{off, g.bkind, g.bsign, 0, g.slot});
+        p->binds.push_back(Bind{off, g.bkind, g.bsign, static_cast<uint16_t>(g.special == SP_BOUND_RZ), g.slot});
     return off;
 }
 
@@ -892,7 +892,10 @@ bool unfix_bound(std::vector<GOp>* gops, std::string* err) {
         if (g.kind == K_DIAG) {
             g.flags &= static_cast<uint8_t>(~F_D1_SPEC);
             g.special = 0;
-            if (g.bkind == QFVM_OP_RZ || g.bkind == QFVM_OP_RZZ) g.flags &= static_cast<uint8_t>(~F_D0_ONE);
+            if (g.bkind == QFVM_OP_RZ || g.bkind == QFVM_OP_RZZ) {
+                g.flags &= static_cast<uint8_t>(~F_D0_ONE);
+                g.special = SP_BOUND_RZ;
+            }
         }
     }
     return true;
