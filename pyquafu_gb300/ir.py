@@ -21,6 +21,8 @@ include/qfvm_gb300.h plus a pool of complex128 matrix entries.
 
 from __future__ import annotations
 
+import math
+
 import numpy as np
 
 # OPMAP (src/qfvm/qasm.hpp:43-46) -> QFVM_OP_* codes of include/qfvm_gb300.h
@@ -81,6 +83,9 @@ OP_DTYPE = np.dtype(
 assert OP_DTYPE.itemsize == 128
 
 
+_NOTHING = ()
+
+
 class Op:
     """One instruction of the packed list (a gate, or a measure/reset/cif)."""
 
@@ -88,19 +93,22 @@ class Op:
                  "qbits", "cbits", "condition", "body")
 
     def __init__(self, name, kind, qubits=(), ncontrols=0, params=(), matrix=None, slot=-1,
-                 qbits=(), cbits=(), condition=0, body=(), gen=None):
+                 qbits=_NOTHING, cbits=_NOTHING, condition=0, body=_NOTHING, gen=None):
         self.name = name
         self.kind = kind
-        self.qubits = tuple(int(q) for q in qubits)
+        self.qubits = tuple(map(int, qubits))
         self.ncontrols = int(ncontrols)
-        self.params = tuple(float(p) for p in params)
+        self.params = tuple(map(float, params))
         self.matrix = matrix
         self.slot = int(slot)
-        self.gen = generator_of(name, kind) if gen is None else int(gen)
-        self.qbits = tuple(int(q) for q in qbits)
-        self.cbits = tuple(int(c) for c in cbits)
+        if gen is None:  # only matrix gates need their name looked at
+            self.gen = GEN_NONE if kind != OP_MATRIX else generator_of(name, kind)
+        else:
+            self.gen = int(gen)
+        self.qbits = qbits if qbits is _NOTHING else tuple(map(int, qbits))
+        self.cbits = cbits if cbits is _NOTHING else tuple(map(int, cbits))
         self.condition = int(condition)
-        self.body = tuple(body)
+        self.body = body if body is _NOTHING else tuple(body)
 
     @property
     def is_gate(self) -> bool:
@@ -140,6 +148,12 @@ def _matrix_of(pyop) -> np.ndarray:
 def read_op(pyop) -> Op | None:
     """from_pyops (instructions.hpp:229-299).  Returns None for dropped ops."""
     name = str(pyop.name).lower()
+    kind = NAMED_KIND.get(name)
+    if kind is not None:
+        pos = pyop.pos
+        if isinstance(pos, (int, np.integer)):
+            pos = (pos,)
+        return Op(name, kind, pos, len(pyop.ctrls) if hasattr(pyop, "ctrls") else 0, pyop._paras)
     if name in SKIPPED:
         return None
     if name == "measure":
@@ -158,8 +172,6 @@ def read_op(pyop) -> Op | None:
     pos = list(pyop.pos) if not isinstance(pyop.pos, (int, np.integer)) else [int(pyop.pos)]
     paras = [float(p) for p in pyop._paras]
     ncontrols = len(pyop.ctrls) if hasattr(pyop, "ctrls") else 0
-    if name in NAMED_KIND:
-        return Op(name, NAMED_KIND[name], pos, ncontrols, paras)
     if name in OPMAP_CLASSIC:  # "creg": named but applies nothing
         return Op(name, OP_NOP, pos, ncontrols, paras)
     return Op(name, OP_MATRIX, pos, ncontrols, paras, matrix=_matrix_of(pyop))
@@ -206,34 +218,42 @@ def validate(ops, num_qubits: int) -> None:
             if op.matrix.shape != (1 << k, 1 << k):
                 raise ValueError(f"{op.name}: matrix shape {op.matrix.shape} does not match {k} targets")
         for p in op.params:
-            if not np.isfinite(p):
+            if not math.isfinite(p):
                 raise ValueError(f"{op.name}: non-finite parameter {p}")
 
 
+_QPAD = [(0,) * (MAX_OP_QUBITS - k) for k in range(MAX_OP_QUBITS + 1)]
+_PPAD = [(0.0,) * (4 - k) for k in range(5)]
+
+
 def pack(ops) -> tuple[np.ndarray, np.ndarray]:
-    """Pack gate ops into (qfvm_op array, complex128 matrix pool)."""
+    """Pack gate ops into (qfvm_op array, complex128 matrix pool).  Column by
+    column: a record field set per gate costs about a microsecond each."""
     gates = [o for o in ops if o.is_gate and o.kind != OP_NOP]
     arr = np.zeros(len(gates), dtype=OP_DTYPE)
     pool = []
-    off = 0
-    for i, o in enumerate(gates):
-        r = arr[i]
-        r["kind"] = o.kind
-        r["ncontrols"] = o.ncontrols
-        r["nqubits"] = len(o.qubits)
-        r["qubits"][: len(o.qubits)] = o.qubits
-        r["slot"] = o.slot
-        r["gen"] = o.gen
-        p = list(o.params)[:4]
-        r["params"][: len(p)] = p
-        if o.matrix is not None:
+    if gates:
+        for o in gates:
+            if len(o.qubits) > MAX_OP_QUBITS:
+                raise ValueError(f"{o.name}: unsupported qubit count {len(o.qubits)}")
+        arr["kind"] = [o.kind for o in gates]
+        arr["ncontrols"] = [o.ncontrols for o in gates]
+        arr["nqubits"] = [len(o.qubits) for o in gates]
+        arr["qubits"] = [o.qubits + _QPAD[len(o.qubits)] for o in gates]
+        arr["slot"] = [o.slot for o in gates]
+        arr["gen"] = [o.gen for o in gates]
+        params = [tuple(o.params)[:4] for o in gates]
+        arr["params"] = [p + _PPAD[len(p)] for p in params]
+        arr["mat_offset"] = -1
+        off = 0
+        for i, o in enumerate(gates):
+            if o.matrix is None:
+                continue
             m = np.ascontiguousarray(o.matrix, dtype=np.complex128)
-            r["mat_dim"] = m.shape[0]
-            r["mat_offset"] = off
+            arr["mat_dim"][i] = m.shape[0]
+            arr["mat_offset"][i] = off
             pool.append(m.ravel())
             off += m.size
-        else:
-            r["mat_offset"] = -1
     pool_arr = np.concatenate(pool) if pool else np.zeros(1, dtype=np.complex128)
     return arr, np.ascontiguousarray(pool_arr, dtype=np.complex128)
 

@@ -90,6 +90,43 @@ def _bitstrings(indices, measures) -> list[str]:
     return [row.tobytes().decode("ascii") for row in chars]
 
 
+def _outcomes(indices, measures) -> tuple[np.ndarray, np.ndarray]:
+    """Distinct measured values, in order of their first shot, and their
+    counts: the integer of a shot's bitstring (character c of nb has weight
+    2^(nb - 1 - c)), without forming the strings."""
+    nb = len(measures)
+    weight = {}
+    for q, c in measures:
+        if c >= nb:
+            # std::string::replace past the end throws in the reference
+            raise QfvmError(f"classical bit {c} outside a {nb}-bit measurement string")
+        weight[c] = q  # a later measure of a classical bit replaces an earlier one
+    idx = np.asarray(indices, dtype=np.uint64)
+    val = np.zeros(idx.size, dtype=np.uint64)
+    for c, q in weight.items():
+        val |= ((idx >> np.uint64(q)) & np.uint64(1)) << np.uint64(nb - 1 - c)
+    vals, first, counts = np.unique(val, return_index=True, return_counts=True)
+    order = np.argsort(first)
+    return vals[order], counts[order]
+
+
+def _count_values(indices, measures) -> dict:
+    """{int(bitstring, 2): count} (qfvm.cpp:95) of the sampled indices."""
+    if len(measures) <= 63 and all(c >= 0 for _, c in measures):
+        vals, counts = _outcomes(indices, measures)
+        return dict(zip(vals.tolist(), counts.tolist()))
+    return {int(s, 2): c for s, c in _count(_bitstrings(indices, measures)).items()}
+
+
+def _count_strings(indices, measures) -> dict:
+    """{bitstring: count} of the sampled indices."""
+    nb = len(measures)
+    if 0 < nb <= 63 and all(c >= 0 for _, c in measures):
+        vals, counts = _outcomes(indices, measures)
+        return {format(v, f"0{nb}b"): c for v, c in zip(vals.tolist(), counts.tolist())}
+    return _count(_bitstrings(indices, measures))
+
+
 def _count(strings) -> dict:
     counts: dict = {}
     for s in strings:
@@ -154,10 +191,9 @@ def simulate_circuit(circuit, inputstate=None, shots=None):
         if shots < 1:
             raise QfvmError("circuits with operations after a measurement need shots >= 1", 1)
         out, final = _shots(n, circ.cbits_num, circ.ops, psi, shots)
-        counts: dict = {}
-        for v in out.tolist():
-            counts[int(v)] = counts.get(int(v), 0) + 1
-        return counts, final
+        vals, first, num = np.unique(out, return_index=True, return_counts=True)
+        order = np.argsort(first)  # in order of their first shot
+        return dict(zip(vals[order].tolist(), num[order].tolist())), final
     if _has_classical(circ.ops):
         # measures only at the end but resets / cifs before them: one
         # trajectory with the measures skipped (simulator.hpp:115-125), then
@@ -174,8 +210,7 @@ def simulate_circuit(circuit, inputstate=None, shots=None):
             uni = _uniforms(shots)
             nat.check(nat.load().qfvm_sampling_statevec(nat.dptr(state.view(np.float64)), state.size,
                                                         nat.dptr(uni), shots, nat.u64ptr(idx)), "sampling")
-            for s_, c in _count(_bitstrings(idx, measures)).items():
-                outcount[int(s_, 2)] = c
+            outcount = _count_values(idx, measures)
         return outcount, state
     ops = _gate_ops(circ.ops)
     ir.validate(ops, n)
@@ -183,11 +218,7 @@ def simulate_circuit(circuit, inputstate=None, shots=None):
     measures = circ.measure_vec
     nshots = shots if measures else 0
     idx = _run(n, ops, state, given, nshots)
-    outcount: dict = {}
-    if measures:
-        for s, c in _count(_bitstrings(idx, measures)).items():
-            outcount[int(s, 2)] = c  # qfvm.cpp:95 stoi(bitstring, 2)
-    return outcount, state
+    return (_count_values(idx, measures) if measures else {}), state
 
 
 def simulate_circuit_gpu(circuit, inputstate=None):
@@ -238,7 +269,7 @@ def sampling_statevec(measures, inputstate, shots):
     rc = nat.load().qfvm_sampling_statevec(nat.dptr(psi.view(np.float64)), psi.size, nat.dptr(uni), shots,
                                           nat.u64ptr(idx))
     nat.check(rc, "sampling_statevec")
-    return _count(_bitstrings(idx, meas))
+    return _count_strings(idx, meas)
 
 
 def expect_statevec(inputstate, paulis):
