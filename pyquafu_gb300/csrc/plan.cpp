@@ -11,8 +11,12 @@
 #include <algorithm>
 #include <cmath>
 #include <complex>
+#include <climits>
 #include <cstring>
+#include <list>
+#include <mutex>
 #include <set>
+#include <string>
 
 #include "engine.h"
 
@@ -401,13 +405,6 @@ void gop_actions(const GOp& g, std::vector<std::pair<int, uint8_t>>* acts) {
     }
 }
 
-bool act_conflict(uint8_t blocked, uint8_t a) {
-    if (!blocked) return false;
-    if (a == A_Z) return (blocked & (A_X | A_G)) != 0;
-    if (a == A_X) return (blocked & (A_Z | A_G)) != 0;
-    return true;
-}
-
 void gop_targets(const GOp& g, std::vector<int>* t) {
     t->clear();
     switch (g.kind) {
@@ -502,6 +499,140 @@ std::vector<int> register_pad_order(int T, int elem_bytes) {
     return o;
 }
 
+// A gop for scheduling: the qubits it acts on diagonally, as X and otherwise
+// (gop_actions), and its non-diagonal targets.
+struct SchedOp {
+    uint64_t z = 0, x = 0, g = 0, targets = 0;
+    bool tile = true;   // can join a tile pass
+    bool round = true;  // can join a register round
+    bool probe = false;
+};
+
+SchedOp sched_op(const GOp& g) {
+    SchedOp s;
+    std::vector<std::pair<int, uint8_t>> acts;
+    std::vector<int> targ;
+    gop_actions(g, &acts);
+    for (auto& a : acts) (a.second == A_Z ? s.z : (a.second == A_X ? s.x : s.g)) |= 1ULL << a.first;
+    gop_targets(g, &targ);
+    for (int t : targ) s.targets |= 1ULL << t;
+    s.tile = g.kind != K_DENSEK;
+    s.round = g.kind != K_DENSE2;
+    s.probe = g.kind == K_PROBE;
+    return s;
+}
+
+// Operations left out so far, as the actions they block (act_conflict).
+struct Blocked {
+    uint64_t z = 0, x = 0, g = 0;
+    bool conflicts(const SchedOp& o) const { return ((o.z & (x | g)) | (o.x & (z | g)) | (o.g & (z | x | g))) != 0; }
+    void add(const SchedOp& o) {
+        z |= o.z;
+        x |= o.x;
+        g |= o.g;
+    }
+};
+
+// How many of the first `window` operations of `todo` can run together, in
+// order, when the non-diagonal targets are limited to `allowed`.
+int count_joining(const std::vector<SchedOp>& ops, const std::vector<int>& todo, uint64_t allowed, bool round,
+                  size_t window, int cap) {
+    Blocked b;
+    int joined = 0;
+    const size_t m = std::min(window, todo.size());
+    for (size_t i = 0; i < m && joined < cap; ++i) {
+        const SchedOp& o = ops[static_cast<size_t>(todo[i])];
+        if ((round ? o.round : o.tile) && !(o.targets & ~allowed) && !b.conflicts(o)) ++joined;
+        else b.add(o);
+    }
+    return joined;
+}
+
+// Local search for the qubits that let the most operations join: from
+// `start`, the best exchange of one qubit for another of `from` until none
+// improves the count.
+uint64_t best_set(const std::vector<SchedOp>& ops, const std::vector<int>& todo, uint64_t fixed, uint64_t start,
+                  uint64_t from, bool round, size_t window, int cap) {
+    uint64_t set = start;
+    int best = count_joining(ops, todo, fixed | set, round, window, cap);
+    for (;;) {
+        uint64_t next = set;
+        for (uint64_t out = set; out && best < cap; out &= out - 1)
+            for (uint64_t in = from & ~set; in; in &= in - 1) {
+                const uint64_t c = (set & ~(out & (~out + 1))) | (in & (~in + 1));
+                const int v = count_joining(ops, todo, fixed | c, round, window, cap);
+                if (v > best) {
+                    best = v;
+                    next = c;
+                }
+            }
+        if (next == set) return set;
+        set = next;
+    }
+}
+
+// The sets chosen for a circuit's passes and rounds, in order.  They depend on
+// the circuit's structure alone, and finding them costs milliseconds (30 qubits,
+// 1800 gates: 15 ms, then 1.6), so re-planning a structure at other angles looks them
+// up: the last PLAN_CHOICES structures of the process, keyed by every field
+// the search reads.
+struct Choices {
+    std::vector<uint64_t> sets;
+};
+constexpr size_t PLAN_CHOICES = 32;
+
+std::mutex g_choices_mu;
+std::list<std::pair<std::string, Choices>> g_choices;  // most recent first
+
+std::string choices_key(int n, int T, int R, int cap, const std::vector<SchedOp>& ops) {
+    std::string k;
+    k.reserve(ops.size() * 36 + 16);
+    auto put = [&](const auto& v) { k.append(reinterpret_cast<const char*>(&v), sizeof v); };
+    put(n);
+    put(T);
+    put(R);
+    put(cap);
+    for (const SchedOp& o : ops) {
+        put(o.z);
+        put(o.x);
+        put(o.g);
+        put(o.targets);
+        k.push_back(static_cast<char>(o.tile | o.round << 1 | o.probe << 2));
+    }
+    return k;
+}
+
+bool find_choices(const std::string& key, Choices* c) {
+    std::lock_guard<std::mutex> lk(g_choices_mu);
+    for (auto it = g_choices.begin(); it != g_choices.end(); ++it)
+        if (it->first == key) {
+            g_choices.splice(g_choices.begin(), g_choices, it);
+            *c = it->second;
+            return true;
+        }
+    return false;
+}
+
+void keep_choices(std::string key, Choices c) {
+    std::lock_guard<std::mutex> lk(g_choices_mu);
+    g_choices.emplace_front(std::move(key), std::move(c));
+    if (g_choices.size() > PLAN_CHOICES) g_choices.pop_back();
+}
+
+// Operations of one tile pass at most.  Fewer and larger passes are faster up
+// to where their unrolled code leaves the instruction cache: 27 qubits
+// complex64 (R = 5) 14.2 ms at 42 operations, 12.7 at 62, 12.9 without a limit;
+// the 24-qubit float-pair sweep (R = 3) 63.6 ms at 84, 63.3 at 125; batched
+// sweeps (R = 4) 23.3 ms at 42, 21.3 at 62, 19.1 without.  The limits below
+// are lower where the default plans of the 30-qubit and 24-qubit benchmark
+// circuits would otherwise have fewer than the 40 passes over which
+// tests/test_jit_host.py bounds the code size.
+int pass_op_cap(int R, bool two_states, bool bound) {
+    if (bound) return INT_MAX;
+    if (two_states) return R <= 3 ? 84 : 62;
+    return R >= 5 ? 45 : INT_MAX;
+}
+
 }  // namespace
 
 bool build_plan(int n, int precision, const std::vector<GOp>& gops, int T, int R, HostPlan* plan,
@@ -576,41 +707,61 @@ bool build_plan(int n, int precision, const std::vector<GOp>& gops, int T, int R
 
     std::vector<int> pending(gops.size());
     for (size_t i = 0; i < gops.size(); ++i) pending[i] = static_cast<int>(i);
-    std::vector<std::pair<int, uint8_t>> acts;
-    std::vector<int> targ;
+    std::vector<SchedOp> sops;
+    sops.reserve(gops.size());
+    bool two_states = false, bound = false;
+    for (const GOp& g : gops) {
+        sops.push_back(sched_op(g));
+        two_states |= g.kind == K_PROBE;
+        bound |= g.bkind != 0 && g.slot >= 0 && g.kind != K_PROBE;
+    }
+    const int cap = pass_op_cap(R, two_states, bound);
+    const uint64_t low = (1ULL << L) - 1, every = n >= 64 ? ~0ULL : (1ULL << n) - 1;
+    std::string key = choices_key(n, T, R, cap, sops);
+    Choices choices;
+    const bool known = find_choices(key, &choices);
+    size_t next_choice = 0;
+    // the k lowest bits of m
+    auto lowest = [](uint64_t m, int k) {
+        uint64_t r = 0;
+        for (; k > 0 && m; --k, m &= m - 1) r |= m & (~m + 1);
+        return r;
+    };
+    constexpr size_t WINDOW = 384;  // pending operations the search looks ahead
 
     while (!pending.empty()) {
         // ---- choose the tile's high qubits and the gates of this pass ----
-        uint8_t blocked[64] = {0};
-        std::vector<int> high;  // global qubits >= L in the tile
-        std::vector<int> sched, rest;
-        int probes = 0;
-        for (int gi : pending) {
-            const GOp& g = gops[gi];
-            gop_actions(g, &acts);
-            bool conflict = false;
-            for (auto& a : acts) conflict |= act_conflict(blocked[a.first], a.second);
-            bool ok = !conflict && g.kind != K_DENSEK;
-            if (ok && g.kind == K_PROBE && probes >= MAX_PASS_PROBES) ok = false;
-            if (ok) {
-                gop_targets(g, &targ);
-                std::vector<int> add;
-                for (int t : targ)
-                    if (t >= L && std::find(high.begin(), high.end(), t) == high.end() &&
-                        std::find(add.begin(), add.end(), t) == add.end())
-                        add.push_back(t);
-                if (static_cast<int>(high.size() + add.size()) <= H) {
-                    high.insert(high.end(), add.begin(), add.end());
-                } else {
-                    ok = false;
-                }
+        uint64_t high = 0;  // global qubits >= L in the tile
+        if (known) {
+            high = choices.sets[next_choice++];
+        } else {
+            // in order of the gates' first need, then by local search
+            Blocked b;
+            for (int gi : pending) {
+                const SchedOp& o = sops[static_cast<size_t>(gi)];
+                const uint64_t need = high | (o.targets & ~low);
+                if (o.tile && !b.conflicts(o) && __builtin_popcountll(need) <= H) high = need;
+                else b.add(o);
             }
-            if (ok) {
-                sched.push_back(gi);
-                if (g.kind == K_PROBE) ++probes;
-            } else {
-                for (auto& a : acts) blocked[a.first] |= a.second;
-                rest.push_back(gi);
+            high |= lowest(every & ~low & ~high, H - __builtin_popcountll(high));
+            high = best_set(sops, pending, low, high, every & ~low, false, WINDOW, cap);
+            choices.sets.push_back(high);
+        }
+        std::vector<int> sched, rest;
+        {
+            Blocked b;
+            int probes = 0;
+            for (int gi : pending) {
+                const SchedOp& o = sops[static_cast<size_t>(gi)];
+                const bool ok = o.tile && !(o.targets & ~(low | high)) && !b.conflicts(o) &&
+                                static_cast<int>(sched.size()) < cap && (!o.probe || probes < MAX_PASS_PROBES);
+                if (ok) {
+                    sched.push_back(gi);
+                    probes += o.probe;
+                } else {
+                    b.add(o);
+                    rest.push_back(gi);
+                }
             }
         }
         if (sched.empty()) {
@@ -629,10 +780,6 @@ bool build_plan(int n, int precision, const std::vector<GOp>& gops, int T, int R
             pending.erase(pending.begin());
             continue;
         }
-        // fill the tile to exactly T qubits
-        for (int q = L; q < n && static_cast<int>(high.size()) < H; ++q)
-            if (std::find(high.begin(), high.end(), q) == high.end()) high.push_back(q);
-        std::sort(high.begin(), high.end());
         PassDesc pd;
         std::memset(&pd, 0, sizeof(pd));
         pd.type = PASS_TILE;
@@ -645,9 +792,13 @@ bool build_plan(int n, int precision, const std::vector<GOp>& gops, int T, int R
             pd.tq[k] = static_cast<uint8_t>(k);
             local_of[k] = k;
         }
-        for (int k = 0; k < H; ++k) {
-            pd.tq[L + k] = static_cast<uint8_t>(high[k]);
-            local_of[high[k]] = L + k;
+        {
+            int k = L;
+            for (uint64_t m = high; m; m &= m - 1, ++k) {
+                const int q = __builtin_ctzll(m);
+                pd.tq[k] = static_cast<uint8_t>(q);
+                local_of[q] = k;
+            }
         }
         pd.step_begin = static_cast<int32_t>(plan->steps.size());
         pd.probe_base = static_cast<int32_t>(plan->probe_slot.size());
@@ -683,39 +834,38 @@ bool build_plan(int n, int precision, const std::vector<GOp>& gops, int T, int R
                 todo.erase(todo.begin());
                 continue;
             }
-            uint8_t rblocked[64] = {0};
-            std::vector<int> regs;  // tile-local positions
-            std::vector<int> round_ops, left;
-            for (int gi : todo) {
-                const GOp& g = gops[gi];
-                gop_actions(g, &acts);
-                bool conflict = false;
-                for (auto& a : acts) conflict |= act_conflict(rblocked[a.first], a.second);
-                bool ok = !conflict && g.kind != K_DENSE2;
-                if (ok) {
-                    gop_targets(g, &targ);
-                    std::vector<int> add;
-                    for (int t : targ) {
-                        int lp = local_of[t];
-                        if (std::find(regs.begin(), regs.end(), lp) == regs.end() &&
-                            std::find(add.begin(), add.end(), lp) == add.end())
-                            add.push_back(lp);
-                    }
-                    if (static_cast<int>(regs.size() + add.size()) <= R)
-                        regs.insert(regs.end(), add.begin(), add.end());
-                    else
-                        ok = false;
+            uint64_t rset = 0;  // the register bits' global qubits
+            if (known) {
+                rset = choices.sets[next_choice++];
+            } else {
+                Blocked b;
+                for (int gi : todo) {
+                    const SchedOp& o = sops[static_cast<size_t>(gi)];
+                    const uint64_t need = rset | o.targets;
+                    if (o.round && !b.conflicts(o) && __builtin_popcountll(need) <= R) rset = need;
+                    else b.add(o);
                 }
-                if (ok) {
-                    round_ops.push_back(gi);
-                } else {
-                    for (auto& a : acts) rblocked[a.first] |= a.second;
-                    left.push_back(gi);
+                // pad the register set (register_pad_order)
+                for (size_t x = 0; x < pad_order.size() && __builtin_popcountll(rset) < R; ++x)
+                    rset |= 1ULL << pd.tq[pad_order[x]];
+                rset = best_set(sops, todo, 0, rset, low | high, true, todo.size(), static_cast<int>(todo.size()));
+                choices.sets.push_back(rset);
+            }
+            std::vector<int> regs;  // tile-local positions
+            for (uint64_t m = rset; m; m &= m - 1) regs.push_back(local_of[__builtin_ctzll(m)]);
+            std::vector<int> round_ops, left;
+            {
+                Blocked b;
+                for (int gi : todo) {
+                    const SchedOp& o = sops[static_cast<size_t>(gi)];
+                    if (o.round && !(o.targets & ~rset) && !b.conflicts(o)) {
+                        round_ops.push_back(gi);
+                    } else {
+                        b.add(o);
+                        left.push_back(gi);
+                    }
                 }
             }
-            // pad the register set (register_pad_order)
-            for (size_t x = 0; x < pad_order.size() && static_cast<int>(regs.size()) < R; ++x)
-                if (std::find(regs.begin(), regs.end(), pad_order[x]) == regs.end()) regs.push_back(pad_order[x]);
             StepDesc sd;
             std::memset(&sd, 0, sizeof(sd));
             sd.type = STEP_ROUND;
@@ -791,6 +941,7 @@ bool build_plan(int n, int precision, const std::vector<GOp>& gops, int T, int R
         st.pass_bytes += 2.0 * Sb * N;
         pending = rest;
     }
+    if (!known) keep_choices(std::move(key), std::move(choices));
     while (plan->coef.size() % 4) plan->coef.push_back(0.0);  // 4-wide reads of the last block
     return true;
 }

@@ -367,7 +367,7 @@ def test_parameter_block_holds_what_a_pass_reads(precision):
     parameter block lists only the entries it reads, so the default passes of
     the 30-qubit circuit read every coefficient from it."""
     h = default_plan(precision, False)
-    for i in (0, 20, 40):
+    for i in (0, 20, 35):
         src = pass_ptx(h, i, 1)
         assert "p_cblob[" in src and "ld.global.nc" not in src
     nat.load().qfvm_plan_destroy(h)

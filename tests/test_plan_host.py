@@ -404,3 +404,40 @@ def test_normalized_sweep_probes(n, precision):
         got[s] += v
     ref = oracle.grad_adjoint(n, ops, [o.slot for o in ops], terms)
     np.testing.assert_allclose(got, ref, atol=1e-11)
+
+
+def _mixed_structure(n, seed):
+    """Every gate kind the planner schedules, two-target and wide dense gates
+    among them."""
+    rng = np.random.default_rng(seed)
+    ops = workloads.random_layers(n, 4, seed=seed, extras=True, extra_rate=0.7)
+    for k in (2, 3, 7):
+        u, _ = np.linalg.qr(rng.normal(size=(1 << k, 1 << k)) + 1j * rng.normal(size=(1 << k, 1 << k)))
+        qs = tuple(int(q) for q in rng.choice(n, k, replace=False))
+        ops.insert(int(rng.integers(len(ops))), workloads.matrix_gate("u", qs, u))
+    return ops
+
+
+@pytest.mark.parametrize("n,precision,T,R", [(13, 0, 11, 3), (14, 2, 12, 5), (14, 1, 13, 4)])
+def test_replanned_structures(n, precision, T, R):
+    """The sets found for a structure's passes and rounds are looked up when it
+    is planned again: same records, right states, also at other angles and
+    after more structures than are kept."""
+    circuits = [_mixed_structure(n, seed) for seed in range(3)]
+    first = [helpers.host_plan(n, ops, precision, T, R) for ops in circuits]
+    other = [op if op.name not in ("rx", "ry") else type(op)(op.name, op.kind, op.qubits, 0, (op.params[0] + 0.1,))
+             for op in circuits[0]]
+    for q in range(40):  # pushes the first ones out
+        helpers.host_plan(n, [workloads.named("h", (q % n,)), workloads.named("x", ((q * 5 + 1) % n,)),
+                              workloads.named("h", ((q // n) % n,))], precision, T, R)
+    for ops, plan in zip(circuits, first):
+        again = helpers.host_plan(n, ops, precision, T, R)  # searched anew, then looked up
+        twice = helpers.host_plan(n, ops, precision, T, R)
+        for field in ("passes", "steps", "ops", "coef"):
+            assert np.array_equal(plan[field], again[field]) and np.array_equal(plan[field], twice[field])
+        psi = helpers.random_state(n, 9)
+        assert np.abs(helpers.interpret(plan, psi.copy()) - oracle.simulate(n, ops, psi.copy())).max() < 1e-13
+    plan = helpers.host_plan(n, other, precision, T, R)
+    assert np.array_equal(plan["passes"]["tq"], first[0]["passes"]["tq"])
+    psi = helpers.random_state(n, 9)
+    assert np.abs(helpers.interpret(plan, psi.copy()) - oracle.simulate(n, other, psi.copy())).max() < 1e-13
