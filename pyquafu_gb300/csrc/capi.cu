@@ -92,8 +92,8 @@ int upload_plan(qfvm_plan* p) {
     if (!hp.ops.empty()) std::memcpy(host.data() + b_pass + b_steps, hp.ops.data(), hp.ops.size() * sizeof(KOp));
     unsigned char* cdst = host.data() + b_pass + b_steps + b_ops;
     if (f32) {
-        float* f = reinterpret_cast<float*>(cdst);
-        for (size_t i = 0; i < hp.coef.size(); ++i) f[i] = static_cast<float>(hp.coef[i]);
+        const std::vector<float> pool = pool_f32(hp);
+        if (!pool.empty()) std::memcpy(cdst, pool.data(), pool.size() * sizeof(float));
     } else if (dsp) {
         float* f = reinterpret_cast<float*>(cdst);
         for (size_t i = 0; i < hp.coef.size(); ++i) {

@@ -269,6 +269,12 @@ void merge_round_diagonals(HostPlan* plan);
 // then costs one multiply-add per real instead of a multiply and a
 // multiply-add, a phase half the amplitudes.  Probes are rescaled to match.
 void normalize_passes(HostPlan* plan);
+// The coefficient pool as complex64 kernels hold it.  Rounded coefficients
+// multiply the state's norm by 1 + O(2^-25) per gate; where nothing is bound
+// later, each gate that scales every amplitude is rounded from coefficients
+// that make up for what the gates before it lost, so the norm is off by one
+// rounding at the end instead of hundreds.
+std::vector<float> pool_f32(const HostPlan& hp);
 // Coefficients of a bindable gate kind at angle th (2 or 4 doubles).
 int bind_coef(int kind, double th, double* c);
 // Gate-equivalent bytes of one gop: 2 * bytes per amplitude * amplitudes it

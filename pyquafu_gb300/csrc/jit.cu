@@ -415,6 +415,7 @@ int prepare_impl(qfvm_plan* p, int nstates, std::string* err) {
     }
     // the coefficient parameter blocks of the compiled passes
     p->jit_cblob[si].assign(hp.passes.size(), {});
+    const std::vector<float> held = hp.arith == QFVM_C64 ? pool_f32(hp) : std::vector<float>();
     for (size_t i = 0; i < hp.passes.size(); ++i) {
         std::vector<uint32_t> entries;
         if (!ks[i] || !jit_pass_coef_block(hp, static_cast<int>(i), sh, &entries)) continue;
@@ -426,9 +427,8 @@ int prepare_impl(qfvm_plan* p, int nstates, std::string* err) {
             const double v = hp.coef[entries[e]];
             unsigned char* d = blob.data() + e * eb;
             if (hp.arith == QFVM_C64) {
-                const float f = static_cast<float>(v);
-                std::memcpy(d, &f, 4);
-                std::memcpy(d + 4, &f, 4);
+                std::memcpy(d, &held[entries[e]], 4);
+                std::memcpy(d + 4, &held[entries[e]], 4);
             } else if (hp.arith == QFVM_C128_DS) {
                 const float h = static_cast<float>(v);
                 const float l = static_cast<float>(v - static_cast<double>(h));

@@ -1311,6 +1311,46 @@ void normalize_passes(HostPlan* plan) {
     }
 }
 
+std::vector<float> pool_f32(const HostPlan& hp) {
+    std::vector<float> out(hp.coef.begin(), hp.coef.end());
+    if (!hp.binds.empty()) return out;
+    double carry = 1.0;  // exact norm over held norm of the ops so far
+    // op's coefficients off .. off + n: scaled by the carry when the op applies
+    // them all to every amplitude; either way the rounding's loss is carried on
+    auto take = [&](uint32_t off, int n, bool absorbs) {
+        const double f = absorbs ? carry : 1.0;
+        double exact = 0.0, held = 0.0;
+        for (int i = 0; i < n; ++i) {
+            const double c = hp.coef[off + i] * f;
+            out[off + i] = static_cast<float>(c);
+            exact += c * c;
+            held += static_cast<double>(out[off + i]) * out[off + i];
+        }
+        if (held <= 0.0) return;
+        carry = (absorbs ? 1.0 : carry) * std::sqrt(exact / held);
+    };
+    auto visit = [&](const KOp& o) {
+        if (o.creg != 0 || (o.kind != K_DIAGR && o.cthr != 0)) return;  // a DIAGR's masks hold its entry codes
+        switch (o.kind) {
+            case K_REAL: take(o.coef, 4, o.special != SP_UNIT); break;
+            case K_RX: take(o.coef, 2, o.special != SP_UNIT); break;
+            case K_DENSE: take(o.coef, 8, true); break;
+            case K_DENSE2: take(o.coef, 32, true); break;
+            case K_DIAG:
+                if (!(o.flags & F_D1_SPEC)) take(o.coef, 4, !(o.flags & F_D0_ONE));
+                break;
+            case K_DIAGR: take(o.coef, 2 << o.k, false); break;
+            default: break;
+        }
+    };
+    for (const PassDesc& pd : hp.passes) {
+        for (int oi = 0; oi < pd.op_count; ++oi) visit(hp.ops[pd.op_begin + oi]);  // whole-state passes, global ops
+        for (int si = pd.step_begin; si < pd.step_begin + pd.step_count; ++si)
+            for (int oi = 0; oi < hp.steps[si].op_count; ++oi) visit(hp.ops[hp.steps[si].op_begin + oi]);
+    }
+    return out;
+}
+
 namespace {
 
 // bits of the register index an op of a round acts on non-diagonally
