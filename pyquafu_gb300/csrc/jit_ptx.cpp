@@ -24,8 +24,10 @@
 // scalar arithmetic and coefficients mostly loaded per thread before:
 // 30 qubits float pairs 1057 -> 939 ms, 27 qubits complex64 20.4 -> 18.2 ms,
 // 24-qubit float-pair gradient 133 -> 101 ms.  With the unit rotations of
-// normalize_passes: 827 ms, 16.5 ms (0.81 of the measured copy bandwidth)
-// and 85 ms; 25 qubits FP64 (bound by the FP64 pipe) 88.0 -> 55.3 ms.
+// normalize_passes: 828 ms, 16.5 ms and 85 ms; 25 qubits FP64 (bound by the
+// FP64 pipe) 88.0 -> 55.3 ms.  With the planner's larger passes: 709 ms,
+// 14.0 ms (35 passes, 0.84 of the measured copy bandwidth each), 54.7 ms; with
+// float pairs renormalised in the last round's registers 679 ms.
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -1290,7 +1292,7 @@ class Gen {
         for (int si = 0; si < pd_.step_count; ++si) {
             const StepDesc& sd = hp_.steps[pd_.step_begin + si];
             if (sd.type == STEP_SMEM) smem_step(sd, base, sbase);
-            else round(sd, base, sbase);
+            else round(sd, base, sbase, out_pair_ && si + 1 == pd_.step_count);
             if (si == 0 && late_next) next_prefetch();
         }
 
@@ -1309,9 +1311,12 @@ class Gen {
             I(fmt("@%s bra %s", pz.c_str(), lskip.c_str()));
             lab(lst);
         }
-        if (out_pair_) {
-            // float pairs for the next pass: renormalised (TwoSum) once here,
-            // so |low| stays within half an ulp of high from pass to pass
+        // float pairs for the next pass: renormalised (TwoSum) once, in the
+        // last round's registers or, after a shared-memory step, here, so that
+        // |low| stays within half an ulp of high from pass to pass
+        const bool round_last = pd_.step_count > 0 &&
+                                hp_.steps[pd_.step_begin + pd_.step_count - 1].type == STEP_ROUND;
+        if (out_pair_ && !round_last) {
             for (int k = 0; k < PER_; ++k)
                 for (int st = 0; st < NS_; ++st) {
                     Cx c = load_amp(tbase, st * tileB_ + sk(k));
@@ -2061,7 +2066,8 @@ class Gen {
         }
     }
 
-    void round(const StepDesc& sd, const std::string& base, const std::string& sbase) {
+    // norm: float pairs leave the round renormalised
+    void round(const StepDesc& sd, const std::string& base, const std::string& sbase, bool norm) {
         round_ = &sd;
         // the thread's tile-layout byte address in this slot; register j adds offb(j)
         std::vector<uint32_t> tsw(T_ - R_);
@@ -2144,6 +2150,9 @@ class Gen {
         if (ph_on_)
             for (int s = 0; s < NS_; ++s)
                 for (int j = 0; j < NA_; ++j) A_[s][j] = phase(A_[s][j], ph_);
+        if (norm)
+            for (int s = 0; s < NS_; ++s)
+                for (int j = 0; j < NA_; ++j) A_[s][j] = cnorm(A_[s][j]);
         // a pending flip of bit t: register j holds logical j ^ (1 << t), whose
         // address is j's plus rsw[t] (bit t of j clear) or minus it (set)
         if (r0 >= 0) materialize(r0);  // pairs are stored as they are

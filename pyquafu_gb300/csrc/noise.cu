@@ -251,13 +251,11 @@ __global__ void __launch_bounds__(256) k_item_sample(const double2* __restrict__
     const uint64_t per = (N + 255) / 256;
     const uint64_t lo = threadIdx.x * per < N ? threadIdx.x * per : N;
     const uint64_t hi = lo + per < N ? lo + per : N;
-    const double r = uni[static_cast<size_t>(item) * ndraws + draw];
-    const double sc = scale[item];  // 1 / the norm the Kraus channels left out (1.0: exact)
+    // the state's norm that the Kraus channels left out is 1 / scale (1.0: exact)
+    const double r = uni[static_cast<size_t>(item) * ndraws + draw] / (scale[item] * scale[item]);
     double s = 0.0;
     for (uint64_t i = lo; i < hi; ++i) {
-        double2 a = st[i];
-        a.x *= sc;
-        a.y *= sc;
+        const double2 a = st[i];
         s = __dadd_rn(s, __dadd_rn(__dmul_rn(a.x, a.x), __dmul_rn(a.y, a.y)));
     }
     sums[threadIdx.x] = s;
@@ -282,9 +280,7 @@ __global__ void __launch_bounds__(256) k_item_sample(const double2* __restrict__
         double cum = base;
         uint64_t pick = N;
         for (uint64_t i = lo; i < hi; ++i) {
-            double2 a = st[i];
-            a.x *= sc;
-            a.y *= sc;
+            const double2 a = st[i];
             cum = __dadd_rn(cum, __dadd_rn(__dmul_rn(a.x, a.x), __dmul_rn(a.y, a.y)));
             if (r < cum) {
                 pick = i;
