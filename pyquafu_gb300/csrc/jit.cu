@@ -264,7 +264,10 @@ JitShape plan_shape(const qfvm_plan* p, int nstates, size_t optin, size_t per_sm
     sh.chain = p->chain_ok ? chain_for(hp, sh) : 0;
     JitShape two_sh = sh;
     two_sh.nb = 2;
-    const size_t two = jit_smem_bytes(hp, two_sh, MAX_PASS_PROBES);
+    size_t cof = 0;
+    for (size_t i = 0; !hp.binds.empty() && i < hp.passes.size(); ++i)
+        cof = std::max(cof, jit_shared_coef_bytes(hp, static_cast<int>(i), two_sh));
+    const size_t two = jit_smem_bytes(hp, two_sh, MAX_PASS_PROBES, cof);
     if (sh.nb == 2 && (two > optin || static_cast<size_t>(sh.minb) * (two + 1024) > per_sm)) sh.nb = 1;
     return sh;
 }
@@ -404,7 +407,7 @@ int prepare_impl(qfvm_plan* p, int nstates, std::string* err) {
         k->threads = nt;
         k->T = hp.T;
         k->entry = jit_entry_name(hp.arith, nstates);
-        k->smem = jit_smem_bytes(hp, sh, np);
+        k->smem = jit_smem_bytes(hp, sh, np, jit_shared_coef_bytes(hp, i, sh));
         if (load(dev, images[w], k.get(), err)) return 1;
         cache().emplace(keys[i], std::move(k));
     }

@@ -47,10 +47,14 @@ bool jit_pass_ptx(const HostPlan& hp, int pi, const JitShape& sh, const std::str
 // when the pass reads them from the pool in global memory.
 bool jit_pass_coef_block(const HostPlan& hp, int pi, const JitShape& sh, std::vector<uint32_t>* entries);
 
+// Bytes of its item's coefficients that pass `pi` keeps in shared memory
+// (plans bound per item on the device; 0: it reads them from global memory or
+// from the parameter block).
+size_t jit_shared_coef_bytes(const HostPlan& hp, int pi, const JitShape& sh);
 // Dynamic shared memory of a specialised pass: nb tile slots of nstates
 // tiles in the padded tile layout, the per-warp probe sums, one mbarrier per
-// slot.
-size_t jit_smem_bytes(const HostPlan& hp, const JitShape& sh, int nprobe);
+// slot, the item's coefficients.
+size_t jit_smem_bytes(const HostPlan& hp, const JitShape& sh, int nprobe, size_t coef_bytes);
 
 // Device status word of the specialised passes (per device, zeroed): a
 // kernel whose bounded wait for its tile copies gave up writes

@@ -28,6 +28,7 @@
 // FP64 pipe) 88.0 -> 55.3 ms.  With the planner's larger passes: 709 ms,
 // 14.0 ms (35 passes, 0.84 of the measured copy bandwidth each), 54.7 ms; with
 // float pairs renormalised in the last round's registers 679 ms.
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -107,6 +108,28 @@ class Gen {
         bulk_out_ = !ds_ || out_pair_;
         if (sh.pcoef) coef_list();
         pc_ = sh.pcoef && !clist_.empty() && blob_bytes() <= kMaxBlob;
+        // Bound per item on the device: a tile's CTA copies its item's
+        // coefficients next to the tile, up to 4 KiB (what one CTA copies in
+        // one or two loads a thread; above it they stay in global memory).
+        // Read from there at each use, they were the largest stall of the
+        // complex64 reverse sweeps: 1024 x 16 qubits, gradients, 19.0 ms
+        // against 18.0 ms with the copy; 2048 x 12 qubits 20.4 against 19.9.
+        // FP64 passes are bound by the FP64 pipe and keep the global reads.
+        if (!f64_ && !hp.binds.empty() && !pc_) {
+            std::vector<uint32_t> used;
+            used.swap(clist_);
+            coef_list();
+            uint32_t hi = 0;
+            slo_ = ~0u;
+            for (uint32_t c : clist_) {
+                slo_ = std::min(slo_, c & ~3u);
+                hi = std::max(hi, c + 1);
+            }
+            sbytes_ = clist_.empty() ? 0 : ((hi + 3u) / 4u * 4u - slo_) * cb_;
+            sc_ = sbytes_ > 0 && sbytes_ <= kMaxShared;
+            if (!sc_) sbytes_ = 0;
+            clist_.swap(used);
+        }
     }
 
     // Coefficient pool entries the pass's operations read, in the order of
@@ -140,6 +163,7 @@ class Gen {
     }
     uint32_t blob_bytes() const { return (static_cast<uint32_t>(clist_.size()) * pb_ + 15u) / 16u * 16u; }
     const std::vector<uint32_t>& coef_entries() const { return clist_; }
+    uint32_t shared_coef_bytes() const { return sbytes_; }
 
     bool param_coefs() const { return pc_; }
     bool in_pairs() const { return in_pair_; }
@@ -836,6 +860,10 @@ class Gen {
     // coefficients off .. off+cnt-1 of the tile's pool (widest aligned loads)
     std::vector<std::string> coefs(uint32_t off, int cnt) {
         if (pc_) return pcoefs(off, cnt);
+        // the pool in global memory, or the item's copy in shared memory
+        const char* space = sc_ ? "shared" : "global.nc";
+        const std::string& basep = sc_ ? cofB_ : coefp_;
+        const uint32_t first = sc_ ? slo_ : 0;
         std::vector<std::string> c;
         uint32_t i = off;
         const uint32_t end = off + cnt;
@@ -843,14 +871,15 @@ class Gen {
             if (ds_) {  // (high, low) float pairs, two per 16-byte load
                 if (i % 2 == 0 && i + 2 <= end) {
                     std::string r[4] = {A(), A(), A(), A()};
-                    I(fmt("ld.global.nc.v4.f32 {%s, %s, %s, %s}, [%s+%u]", r[0].c_str(), r[1].c_str(),
-                          r[2].c_str(), r[3].c_str(), coefp_.c_str(), i * cb_));
+                    I(fmt("ld.%s.v4.f32 {%s, %s, %s, %s}, [%s+%u]", space, r[0].c_str(), r[1].c_str(),
+                          r[2].c_str(), r[3].c_str(), basep.c_str(), (i - first) * cb_));
                     c.push_back(r[0] + "|" + r[1]);
                     c.push_back(r[2] + "|" + r[3]);
                     i += 2;
                 } else {
                     std::string h = A(), l = A();
-                    I(fmt("ld.global.nc.v2.f32 {%s, %s}, [%s+%u]", h.c_str(), l.c_str(), coefp_.c_str(), i * cb_));
+                    I(fmt("ld.%s.v2.f32 {%s, %s}, [%s+%u]", space, h.c_str(), l.c_str(), basep.c_str(),
+                          (i - first) * cb_));
                     c.push_back(h + "|" + l);
                     ++i;
                 }
@@ -862,13 +891,13 @@ class Gen {
             std::string r[4];
             for (int k = 0; k < vec; ++k) r[k] = A();
             if (vec == 4)
-                I(fmt("ld.global.nc.v4.f32 {%s, %s, %s, %s}, [%s+%u]", r[0].c_str(), r[1].c_str(), r[2].c_str(),
-                      r[3].c_str(), coefp_.c_str(), i * cb_));
+                I(fmt("ld.%s.v4.f32 {%s, %s, %s, %s}, [%s+%u]", space, r[0].c_str(), r[1].c_str(), r[2].c_str(),
+                      r[3].c_str(), basep.c_str(), (i - first) * cb_));
             else if (vec == 2)
-                I(fmt("ld.global.nc.v2.%s {%s, %s}, [%s+%u]", ft_, r[0].c_str(), r[1].c_str(), coefp_.c_str(),
-                      i * cb_));
+                I(fmt("ld.%s.v2.%s {%s, %s}, [%s+%u]", space, ft_, r[0].c_str(), r[1].c_str(), basep.c_str(),
+                      (i - first) * cb_));
             else
-                I(fmt("ld.global.nc.%s %s, [%s+%u]", ft_, r[0].c_str(), coefp_.c_str(), i * cb_));
+                I(fmt("ld.%s.%s %s, [%s+%u]", space, ft_, r[0].c_str(), basep.c_str(), (i - first) * cb_));
             for (int k = 0; k < vec; ++k) c.push_back(r[k]);
             i += vec;
         }
@@ -981,7 +1010,7 @@ class Gen {
             // bounds of the checked accesses: the dynamic shared memory, and
             // each state (ntiles tiles of 2^T amplitudes)
             smend_ = R32();
-            Iraw(fmt("add.u32 %s, %s, %u", smend_.c_str(), smb_.c_str(), mbar_off() + 8u * sh_.nb));
+            Iraw(fmt("add.u32 %s, %s, %u", smend_.c_str(), smb_.c_str(), cof_off() + sbytes_));
             std::string nb = R64();
             Iraw(fmt("shl.b64 %s, %s, %d", nb.c_str(), ntiles_.c_str(), T_));
             std::string bytes = R64();
@@ -1035,6 +1064,8 @@ class Gen {
         // any copy of that phase is issued
         mbarB_ = R32();
         I(fmt("add.u32 %s, %s, %u", mbarB_.c_str(), smb_.c_str(), mbar_off()));
+        cofB_ = R32();
+        I(fmt("add.u32 %s, %s, %u", cofB_.c_str(), smb_.c_str(), cof_off()));
         t0_ = P();
         I(fmt("setp.eq.u32 %s, %s, 0", t0_.c_str(), tid_.c_str()));
         {
@@ -1110,6 +1141,8 @@ class Gen {
     uint32_t srun(uint32_t r) const { return tile_off(r << TILE_RUN_BITS, padu_) * es_; }
     // shared byte offset of the mbarriers: after the slots and the probe sums
     uint32_t mbar_off() const { return slotB_ * sh_.nb + static_cast<uint32_t>(NW_ * np_ * 8); }
+    // and of the item's coefficients, after them
+    uint32_t cof_off() const { return (mbar_off() + 8u * sh_.nb + 15u) / 16u * 16u; }
     std::string gaddr_off(const std::string& gp, uint64_t off) {
         if (off < (1ULL << 31)) return gp + "+" + std::to_string(off);
         std::string a = R64();
@@ -1229,6 +1262,24 @@ class Gen {
         I(fmt("mul.lo.u64 %s, %s, %s", coff.c_str(), item.c_str(), cstrideB_.c_str()));
         coefp_ = R64();
         I(fmt("add.s64 %s, %s, %s", coefp_.c_str(), coef0_.c_str(), coff.c_str()));
+        if (sc_) {
+            // the item's coefficients of this pass, 16 bytes a thread: every
+            // thread is past the last tile's reads (the barrier at its end), and
+            // the barrier of the tile's wait comes before this tile's
+            const int vecs = static_cast<int>(sbytes_ / 16u);
+            std::string t64 = R64(), src = R64(), dst = R32();
+            I(fmt("mul.wide.u32 %s, %s, 16", t64.c_str(), tid_.c_str()));
+            I(fmt("add.s64 %s, %s, %s", src.c_str(), coefp_.c_str(), t64.c_str()));
+            I(fmt("mad.lo.u32 %s, %s, 16, %s", dst.c_str(), tid_.c_str(), cofB_.c_str()));
+            for (int v0 = 0; v0 < vecs; v0 += NT_) {
+                std::string p = P(), r[4] = {A(), A(), A(), A()};
+                I(fmt("setp.lt.u32 %s, %s, %d", p.c_str(), tid_.c_str(), vecs - v0));
+                I(fmt("@%s ld.global.nc.v4.f32 {%s, %s, %s, %s}, [%s+%u]", p.c_str(), r[0].c_str(), r[1].c_str(),
+                      r[2].c_str(), r[3].c_str(), src.c_str(), slo_ * cb_ + 16u * static_cast<uint32_t>(v0)));
+                I(fmt("@%s st.shared.v4.f32 [%s+%u], {%s, %s, %s, %s}", p.c_str(), dst.c_str(),
+                      16u * static_cast<uint32_t>(v0), r[0].c_str(), r[1].c_str(), r[2].c_str(), r[3].c_str()));
+            }
+        }
         std::string sbase = R32();
         I(fmt("add.u32 %s, %s, %s", sbase.c_str(), smb_.c_str(), slot.c_str()));
         I(fmt("mad.lo.u32 %s, %s, 8, %s", cmbar.c_str(), sidx.c_str(), mbarB_.c_str()));
@@ -2224,6 +2275,10 @@ class Gen {
     std::map<uint32_t, uint32_t> cindex_;    // pool entry -> its place there
     static constexpr uint32_t kMaxBlob = 24576;  // bytes of coefficients in the kernel parameters
     uint32_t pb_;                                // bytes of one of them
+    static constexpr uint32_t kMaxShared = 4096;  // bytes of an item's coefficients in shared memory
+    bool sc_ = false;                             // coefficients copied to shared memory tile by tile:
+    uint32_t slo_ = 0, sbytes_ = 0;               // pool entries from slo_ on, so many bytes
+    std::string cofB_;
     std::map<std::string, std::string> both_, negc_;
     std::map<std::string, uint32_t> param_at_;  // parameter-block offset of a coefficient
     std::map<std::string, Cx> turned_;
@@ -2276,6 +2331,7 @@ bool jit_pass_key(const HostPlan& hp, int pi, const JitShape& sh, std::string* k
     put(&k, sh.nb);
     put(&k, sh.minb);
     put(&k, static_cast<int>(g.param_coefs()));
+    put(&k, g.shared_coef_bytes());
     put(&k, sh.bounds);
     put(&k, static_cast<int>(g.in_pairs()));
     put(&k, static_cast<int>(g.out_pairs()));
@@ -2320,12 +2376,17 @@ bool jit_pass_coef_block(const HostPlan& hp, int pi, const JitShape& sh, std::ve
     return true;
 }
 
-size_t jit_smem_bytes(const HostPlan& hp, const JitShape& sh, int nprobe) {
+size_t jit_shared_coef_bytes(const HostPlan& hp, int pi, const JitShape& sh) {
+    return hp.passes[pi].type == PASS_TILE ? Gen(hp, pi, sh).shared_coef_bytes() : 0;
+}
+
+size_t jit_smem_bytes(const HostPlan& hp, const JitShape& sh, int nprobe, size_t coef_bytes) {
     const int es = hp.arith == QFVM_C64 ? 8 : 16;
     const size_t tileB = static_cast<size_t>(tile_elems(hp.T, es)) * es;
     const size_t nw = static_cast<size_t>(1 << (hp.T - hp.R)) / 32;
     const size_t np = sh.nstates == 2 ? static_cast<size_t>(nprobe) : 0;
-    return static_cast<size_t>(sh.nb) * sh.nstates * tileB + nw * np * 8 + 8 * static_cast<size_t>(sh.nb);
+    const size_t base = static_cast<size_t>(sh.nb) * sh.nstates * tileB + nw * np * 8 + 8 * static_cast<size_t>(sh.nb);
+    return coef_bytes ? (base + 15) / 16 * 16 + coef_bytes : base;
 }
 
 bool jit_pass_ptx(const HostPlan& hp, int pi, const JitShape& sh, const std::string& entry, std::string* ptx,

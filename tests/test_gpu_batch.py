@@ -176,3 +176,23 @@ def test_observable_forms(n, precision):
             ev, g = bs.run([vals], grads=True)
             np.testing.assert_allclose(ev[0][:, 0], ref_e[:, k], atol=tol)
             np.testing.assert_allclose(g[0][1][mask], ref_grad(1, o)[mask], atol=tol)
+
+
+@pytest.mark.parametrize("precision", ["c64", "c128_ds"])
+@pytest.mark.parametrize("n,layers", [(14, 1), (14, 10)])
+def test_bound_coefficient_ranges(precision, n, layers):
+    """Items of several tiles with their own angles, in passes whose
+    coefficients fit a CTA's copy in shared memory and in larger ones; more
+    items than resident CTAs, so that a CTA changes items between tiles."""
+    vtol, gtol = TOL[precision]
+    ops, nslots = encoded_hea(n, layers, seed=layers)
+    terms = [(1.0, "Z", [0])]
+    items = 200
+    vals = np.random.default_rng(layers).uniform(-np.pi, np.pi, (items, nslots))
+    with BatchSession(precision, grads=True) as bs:
+        bs.add_group(n, ops, terms, items, nslots)
+        ev, g = bs.run([vals], grads=True)
+    for i in (0, 1, 101, items - 1):
+        e, ge = oracle_item(n, ops, vals[i], terms)
+        assert abs(ev[0][i, 0] - e) < vtol
+        np.testing.assert_allclose(g[0][i], ge, atol=gtol)

@@ -388,3 +388,42 @@ def test_float_pair_products_are_rounded():
     for q in re.findall(r"mul\.rn\.f32x2 (%q\d+),", src):
         uses = re.findall(rf"\n\t(\S+) %q\d+, [^;]*{q}[,;]", src)
         assert uses and all(u == "fma.rn.f32x2" for u in uses), (q, uses)
+
+
+@pytest.mark.parametrize("precision", [nat.QFVM_C64, nat.QFVM_C128_DS])
+@pytest.mark.parametrize("layers", [1, 12])
+def test_bound_coefficients_in_shared_memory(precision, layers):
+    """A pass of a plan bound per item copies its pool range to shared memory
+    when that takes at most 4 KiB, and reads nothing else from the pool; a
+    larger range, and every FP64 pass, stays in global memory."""
+    import re
+
+    ops, _ = workloads.hea(16, layers, seed=1, encode=np.zeros(16))
+    size = 4 if precision == nat.QFVM_C64 else 8
+    seen = set()
+    for prec in (precision, nat.QFVM_C128):
+        for adjoint in (False, True):
+            h = plan_handle(16, ops, prec, batched=True, adjoint=adjoint)
+            counts, shape = (ctypes.c_int64 * 4)(), (ctypes.c_int32 * 3)()
+            nat.load().qfvm_plan_host_counts(h, counts, shape)
+            for i in range(counts[0]):
+                src = pass_ptx(h, i, 2 if adjoint else 1)
+                if src is None:
+                    continue
+                copies = re.findall(r"@%\w+ ld\.global\.nc\.v4\.f32 [^\[]*\[[^+\]]*\+(\d+)\]", src)
+                reads = re.findall(r"(?m)^\s*ld\.global\.nc\.(?:v[24]\.)?f(?:32|64)", src)
+                if prec == nat.QFVM_C128:
+                    assert not copies
+                    continue
+                assert not (copies and reads)
+                if not (copies or reads):
+                    continue
+                seen.add(bool(copies))
+                if copies:
+                    assert all(int(c) % 16 == 0 for c in copies)
+                    threads = int(re.search(r"\.(?:max|req)ntid (\d+)", src).group(1))
+                    assert (len(copies) - 1) * threads * 16 < 4096
+            nat.load().qfvm_plan_destroy(h)
+    assert True in seen
+    if layers == 12 and size == 8:
+        assert False in seen
