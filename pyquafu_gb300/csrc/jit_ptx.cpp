@@ -26,8 +26,10 @@
 // 24-qubit float-pair gradient 133 -> 101 ms.  With the unit rotations of
 // normalize_passes: 828 ms, 16.5 ms and 85 ms; 25 qubits FP64 (bound by the
 // FP64 pipe) 88.0 -> 55.3 ms.  With the planner's larger passes: 709 ms,
-// 14.0 ms (35 passes, 0.84 of the measured copy bandwidth each), 54.7 ms; with
-// float pairs renormalised in the last round's registers 679 ms.
+// 14.0 ms (35 passes, 0.79 of the measured copy bandwidth each), 54.7 ms; with
+// float pairs renormalised in the last round's registers 679 ms.  The 24-qubit
+// gradient: 62.5 ms with the larger passes, 54.7 ms with probe sums in float
+// pairs.
 #include <algorithm>
 #include <cstdarg>
 #include <cstdio>
