@@ -1188,16 +1188,26 @@ void simplify_plain(std::vector<GOp>* gops) {
 
 namespace {
 
-// Scalars taken out of a pass's gates (normalize_passes): at most
-// NORM_GROUP in a row before one gate takes their product back.  A gate is
-// left as it is where its scalar is below 2^-24 or the group has already
-// taken out 2^-64 (amplitudes grow by the inverse until the scalar is put
-// back, and float pairs need the range below them).  At random angles a
-// scalar is about 1/2 in the geometric mean and both limits are next to
-// never met (4e-8 per gate, below 1e-9 per group), so that passes which
-// differ only in their angles stay alike and share one compiled kernel.
-constexpr int NORM_GROUP = 16;
-constexpr double NORM_MIN = 0x1p-24, NORM_TOTAL = 0x1p-64;
+// Scalars taken out of a pass's gates (normalize_passes): at most `count` in
+// a row before one gate takes their product back, and down to `total`.
+// Amplitudes grow by the inverse until the scalar is put back (and shrink by
+// as much where the gate that takes it comes first), so the limits keep them
+// and the low halves of float pairs inside FP32's exponents (2^-149 to 2^128):
+//   one state: 2^48 leaves a factor of 2^80 to an input state far from
+//     normalised, and to Hadamards without their 1/sqrt(2);
+//   reverse sweep: a probe multiplies two states and its coefficient is
+//     divided by the square: 2^64 leaves as much to an observable, and a
+//     coefficient's low half is 2^-113 then.
+// A gate whose scalar is below NORM_MIN is left as it is.  At random angles a
+// scalar is about 1/2 in the geometric mean and the limits are seldom met
+// (4e-8 per gate, 4e-6 and 6e-6 per group), so that passes which differ only
+// in their angles stay alike and share one compiled kernel.
+struct NormLimits {
+    int count;
+    double total;
+};
+constexpr NormLimits NORM_ONE_STATE = {15, 0x1p-48}, NORM_SWEEP = {7, 0x1p-32};
+constexpr double NORM_MIN = 0x1p-24;
 
 bool uncontrolled(const KOp& o) { return o.cthr == 0 && o.creg == 0; }
 
@@ -1248,6 +1258,7 @@ void normalize_passes(HostPlan* plan) {
         std::vector<int> ops;  // in execution order
         for (int si = pd.step_begin; si < pd.step_begin + pd.step_count; ++si)
             for (int oi = 0; oi < plan->steps[si].op_count; ++oi) ops.push_back(plan->steps[si].op_begin + oi);
+        const NormLimits lim = pd.nprobe > 0 ? NORM_SWEEP : NORM_ONE_STATE;
         std::vector<double> z2(ops.size(), 1.0);  // factor on |state|^2 from this op on
         for (size_t i0 = 0, i1 = 0; i0 < ops.size(); i0 = i1) {
             // the group, and the op of it that takes the product of the scalars
@@ -1256,7 +1267,7 @@ void normalize_passes(HostPlan* plan) {
             size_t keeper = ops.size(), last_diag = ops.size(), last_rot = ops.size();
             int count = 0;
             cd f;
-            for (i1 = i0; i1 < ops.size() && count <= NORM_GROUP; ++i1) {
+            for (i1 = i0; i1 < ops.size() && count <= lim.count; ++i1) {
                 const KOp& o = plan->ops[ops[i1]];
                 if (free_scalar_coefs(o, pd.nprobe > 0)) keeper = i1;
                 if (!scalar_of(o, plan->coef.data() + o.coef, &f)) continue;
@@ -1269,7 +1280,7 @@ void normalize_passes(HostPlan* plan) {
             for (size_t i = i0; i < i1; ++i) {
                 KOp& o = plan->ops[ops[i]];
                 double* c = plan->coef.data() + o.coef;
-                if (i == keeper || !scalar_of(o, c, &f) || std::abs(total * f) < NORM_TOTAL) continue;
+                if (i == keeper || !scalar_of(o, c, &f) || std::abs(total * f) < lim.total) continue;
                 total *= f;
                 z2[i] /= std::norm(f);
                 if (o.kind == K_REAL) {

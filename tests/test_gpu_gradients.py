@@ -151,3 +151,26 @@ def test_input_state_gradient():
     ref = oracle.grad_adjoint(n, ops, [o.slot for o in ops], terms, psi_in=psi)
     _, g = gradients.adjoint(n, ops, terms, "c128", psi=psi)
     np.testing.assert_allclose(g, ref, atol=1e-10)
+
+
+@pytest.mark.parametrize("precision,tol", [("c128_ds", 1e-10), ("c64", 1e-5)])
+@pytest.mark.parametrize("angles", ["spread", "equal", "eps"])
+@pytest.mark.parametrize("rz", [False, True])
+def test_trained_angles(precision, tol, angles, rz):
+    """Angles near 0 and pi, where a rotation's cosine is small: the products
+    of a sweep's probes stay finite and keep the digits they have at uniform
+    angles (same tolerances)."""
+    n, rng = 14, np.random.default_rng(5)
+    ops, params = workloads.hea(n, 4, seed=n)
+    ops = [o for o in ops if rz or o.name != "rz"]
+    rotations = [o for o in ops if o.slot >= 0]
+    k = len(rotations)
+    th = {"spread": rng.integers(0, 2, k) * np.pi + rng.normal(0, 1e-3, k), "equal": np.full(k, 3.0157),
+          "eps": np.full(k, np.pi - 3.2e-4)}[angles]
+    for i, o in enumerate(rotations):
+        o.params, o.slot = (float(th[i]),), i
+    terms = workloads.zz_x_hamiltonian(n, seed=n)
+    ref = oracle.grad_adjoint(n, ops, [o.slot for o in ops], terms)
+    e, g = gradients.adjoint(n, ops, terms, precision)
+    assert abs(e - oracle.energy(n, ops, terms)) < tol
+    np.testing.assert_allclose(g, ref, atol=tol)

@@ -441,3 +441,58 @@ def test_replanned_structures(n, precision, T, R):
     assert np.array_equal(plan["passes"]["tq"], first[0]["passes"]["tq"])
     psi = helpers.random_state(n, 9)
     assert np.abs(helpers.interpret(plan, psi.copy()) - oracle.simulate(n, other, psi.copy())).max() < 1e-13
+
+
+def _trained_angles(kind, count, seed):
+    """Angles of trained and initialised circuits: all equal, or each 0 or pi
+    with a spread."""
+    rng = np.random.default_rng(seed)
+    if kind.startswith("spread"):
+        return rng.integers(0, 2, count) * np.pi + rng.normal(0, float(kind[6:]), count)
+    return np.full(count, np.pi - float(kind[4:]) if kind.startswith("eps") else float(kind[5:]))
+
+
+def _trained_circuit(n, layers, ansatz, kind, seed=0):
+    ops, params = workloads.hea(n, layers, seed=seed)
+    if ansatz == "ry":
+        ops = [o for o in ops if o.name != "rz"]
+    rotations = [o for o in ops if o.name in ("ry", "rz")]
+    for k, (o, a) in enumerate(zip(rotations, _trained_angles(kind, len(rotations), seed))):
+        o.params, o.slot = (float(a),), k
+    return ops
+
+
+@pytest.mark.parametrize("precision", [1, 2])
+@pytest.mark.parametrize("ansatz,n,layers", [("ry", 13, 4), ("ryrz", 14, 2)])
+@pytest.mark.parametrize("kind", ["spread1e-1", "spread1e-3", "equal3.0157", "equal3.1337", "equal3.1403", "eps 3.2e-4",
+                                  "eps 1e-6"])
+def test_sweep_probes_stay_in_single_precision(monkeypatch, precision, ansatz, n, layers, kind):
+    """A reverse sweep's probes meet both states while scalars of its pass are
+    out: their products and the probe's coefficient, divided by the square,
+    have to stay within FP32's exponents, also for an observable of 1e3 times
+    the size and with the low half of a float pair (48 bits below)."""
+    ops = _trained_circuit(n, layers, ansatz, kind, seed=n)
+    terms = [(1e3 * c, p, q) for c, p, q in workloads.zz_x_hamiltonian(n, seed=n)]
+    plan = helpers.host_plan(n, ops, precision, adjoint=True)
+    worst = []
+    inner = helpers.probe_value
+
+    def probe(psi, lam, xmask, zmask, cmask, ny, scale):
+        ix = np.arange(psi.size) ^ xmask
+        products = np.abs(psi[ix]) * np.abs(lam)
+        high = np.float32(scale)
+        pair = float(high) + float(np.float32(scale - float(high)))
+        worst.append((products.sum(), abs(pair / scale - 1), abs(scale)))
+        return inner(psi, lam, xmask, zmask, cmask, ny, scale)
+
+    monkeypatch.setattr(helpers, "probe_value", probe)
+    psi = oracle.simulate(n, ops)
+    vals = helpers.interpret2(plan, psi, oracle.apply_hamiltonian(psi, terms))
+    products, pair, scale = (max(w[k] for w in worst) for k in range(3))
+    # sums of products: |psi| |lam| <= 1e3 * sum |c| < 2^16, taken out: 2^-32 of each state
+    assert products < 2.0 ** 80 and scale < 2.0 ** 80
+    assert pair < 2.0 ** -46
+    got = np.zeros(max(o.slot for o in ops) + 1)
+    for v, s in zip(vals, plan["probe_slots"]):
+        got[s] += v
+    np.testing.assert_allclose(got, oracle.grad_adjoint(n, ops, [o.slot for o in ops], terms), atol=1e-8)
