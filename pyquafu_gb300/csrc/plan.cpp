@@ -1198,10 +1198,16 @@ namespace {
 //   reverse sweep: a probe multiplies two states and its coefficient is
 //     divided by the square: 2^64 leaves as much to an observable, and a
 //     coefficient's low half is 2^-113 then.
-// A gate whose scalar is below NORM_MIN is left as it is.  At random angles a
-// scalar is about 1/2 in the geometric mean and the limits are seldom met
-// (4e-8 per gate, 4e-6 and 6e-6 per group), so that passes which differ only
-// in their angles stay alike and share one compiled kernel.
+// A gate whose scalar is below NORM_MIN is left as it is.
+//
+// Passes that differ only in their angles have to share one compiled kernel,
+// and a kernel depends on which gates are in unit form.  So every group of a
+// pass gives up all its scalars but one, or, where a group's product is beyond
+// the limit, every second rotation of the pass its own: two patterns a pass
+// (gate by gate up to the limit, a circuit near pi met new patterns at almost
+// every step of a training).  At random angles a scalar is about 1/2 in the
+// geometric mean: 4e-8 of the gates are below NORM_MIN, 4e-6 and 6e-6 of the
+// groups beyond their limit.
 struct NormLimits {
     int count;
     double total;
@@ -1226,7 +1232,7 @@ bool scalar_of(const KOp& o, const double* c, cd* f) {
     } else {
         return false;
     }
-    return std::abs(*f) >= NORM_MIN;
+    return std::abs(*f) >= NORM_MIN && std::abs(*f) <= 1.0 / NORM_MIN;
 }
 
 // number of (complex) coefficients a scalar multiplies into at no cost: the
@@ -1249,6 +1255,56 @@ void scale_complex(double* c, int n, cd z) {
     }
 }
 
+// ops: a pass's operations in order; `from`: some of them with a scalar
+cd product_of_scalars(HostPlan* plan, const std::vector<int>& ops, const std::vector<size_t>& from, size_t keeper) {
+    cd total(1.0, 0.0), f;
+    for (size_t i : from)
+        if (i != keeper && scalar_of(plan->ops[ops[i]], plan->coef.data() + plan->ops[ops[i]].coef, &f)) total *= f;
+    return total;
+}
+
+bool in_range(cd z, double least) { return std::abs(z) >= least && std::abs(z) <= 1.0 / least; }
+
+// Takes the scalars of `from` (but the keeper's) out and multiplies the keeper
+// by their product; z2: the factors on |state|^2 from each operation on.
+void move_scalars(HostPlan* plan, const std::vector<int>& ops, const std::vector<size_t>& from, size_t keeper,
+                  std::vector<double>* z2) {
+    const cd total = product_of_scalars(plan, ops, from, keeper);
+    cd f;
+    for (size_t i : from) {
+        KOp& o = plan->ops[ops[i]];
+        double* c = plan->coef.data() + o.coef;
+        if (i == keeper || !scalar_of(o, c, &f)) continue;
+        (*z2)[i] /= std::norm(f);
+        if (o.kind == K_REAL) {
+            c[1] /= c[0];
+            c[2] /= c[0];
+            c[0] = c[3] = 1.0;
+            o.special = SP_UNIT;
+        } else if (o.kind == K_RX) {
+            c[1] /= c[0];
+            c[0] = 1.0;
+            o.special = SP_UNIT;
+        } else {
+            const cd d1 = cd(c[2], c[3]) / f;
+            c[0] = 1.0;
+            c[1] = 0.0;
+            c[2] = d1.real();
+            c[3] = d1.imag();
+            o.flags |= F_D0_ONE;
+        }
+    }
+    if (total == cd(1.0, 0.0)) return;
+    const KOp& o = plan->ops[ops[keeper]];
+    double* c = plan->coef.data() + o.coef;
+    if (o.kind == K_REAL || o.kind == K_RX) {
+        for (int i = 0; i < (o.kind == K_REAL ? 4 : 2); ++i) c[i] *= total.real();
+    } else {
+        scale_complex(c, o.kind == K_DIAG ? 2 : free_scalar_coefs(o, false), total);
+    }
+    (*z2)[keeper] *= std::norm(total);
+}
+
 }  // namespace
 
 void normalize_passes(HostPlan* plan) {
@@ -1260,56 +1316,41 @@ void normalize_passes(HostPlan* plan) {
             for (int oi = 0; oi < plan->steps[si].op_count; ++oi) ops.push_back(plan->steps[si].op_begin + oi);
         const NormLimits lim = pd.nprobe > 0 ? NORM_SWEEP : NORM_ONE_STATE;
         std::vector<double> z2(ops.size(), 1.0);  // factor on |state|^2 from this op on
+        // the groups, and the op of each that takes the product of the scalars
+        // back: one that does so at no cost, else a phase that stays in its
+        // full form, else (the product is then real) a rotation
+        struct Group {
+            std::vector<size_t> diags, rots;
+            size_t keeper;
+        };
+        std::vector<Group> groups;
+        bool within = true;
         for (size_t i0 = 0, i1 = 0; i0 < ops.size(); i0 = i1) {
-            // the group, and the op of it that takes the product of the scalars
-            // back: one that does so at no cost, else a phase that stays in
-            // its full form, else (the product is then real) a rotation
-            size_t keeper = ops.size(), last_diag = ops.size(), last_rot = ops.size();
-            int count = 0;
+            Group g{{}, {}, ops.size()};
             cd f;
-            for (i1 = i0; i1 < ops.size() && count <= lim.count; ++i1) {
+            for (i1 = i0; i1 < ops.size() && static_cast<int>(g.diags.size() + g.rots.size()) <= lim.count; ++i1) {
                 const KOp& o = plan->ops[ops[i1]];
-                if (free_scalar_coefs(o, pd.nprobe > 0)) keeper = i1;
-                if (!scalar_of(o, plan->coef.data() + o.coef, &f)) continue;
-                (o.kind == K_DIAG ? last_diag : last_rot) = i1;
-                ++count;
+                if (free_scalar_coefs(o, pd.nprobe > 0)) g.keeper = i1;
+                if (scalar_of(o, plan->coef.data() + o.coef, &f)) (o.kind == K_DIAG ? g.diags : g.rots).push_back(i1);
             }
-            if (keeper == ops.size()) keeper = last_diag < ops.size() ? last_diag : last_rot;
-            if (keeper == ops.size()) continue;
-            cd total(1.0, 0.0);
-            for (size_t i = i0; i < i1; ++i) {
-                KOp& o = plan->ops[ops[i]];
-                double* c = plan->coef.data() + o.coef;
-                if (i == keeper || !scalar_of(o, c, &f) || std::abs(total * f) < lim.total) continue;
-                total *= f;
-                z2[i] /= std::norm(f);
-                if (o.kind == K_REAL) {
-                    c[1] /= c[0];
-                    c[2] /= c[0];
-                    c[0] = c[3] = 1.0;
-                    o.special = SP_UNIT;
-                } else if (o.kind == K_RX) {
-                    c[1] /= c[0];
-                    c[0] = 1.0;
-                    o.special = SP_UNIT;
-                } else {
-                    const cd d1 = cd(c[2], c[3]) / f;
-                    c[0] = 1.0;
-                    c[1] = 0.0;
-                    c[2] = d1.real();
-                    c[3] = d1.imag();
-                    o.flags |= F_D0_ONE;
-                }
+            if (g.diags.empty() && g.rots.empty()) continue;
+            if (g.keeper == ops.size()) g.keeper = !g.diags.empty() ? g.diags.back() : g.rots.back();
+            within &= in_range(product_of_scalars(plan, ops, g.rots, g.keeper) *
+                                   product_of_scalars(plan, ops, g.diags, g.keeper), lim.total);
+            groups.push_back(std::move(g));
+        }
+        for (const Group& g : groups) {
+            if (within) {
+                std::vector<size_t> all = g.diags;
+                all.insert(all.end(), g.rots.begin(), g.rots.end());
+                move_scalars(plan, ops, all, g.keeper, &z2);
+                continue;
             }
-            if (total == cd(1.0, 0.0)) continue;
-            const KOp& o = plan->ops[ops[keeper]];
-            double* c = plan->coef.data() + o.coef;
-            if (o.kind == K_REAL || o.kind == K_RX) {
-                for (int i = 0; i < (o.kind == K_REAL ? 4 : 2); ++i) c[i] *= total.real();
-            } else {
-                scale_complex(c, o.kind == K_DIAG ? 2 : free_scalar_coefs(o, false), total);
-            }
-            z2[keeper] *= std::norm(total);
+            // a phase's scalar is 1 in magnitude where the gate is unitary, a
+            // rotation's NORM_MIN at least
+            if (!g.diags.empty() && in_range(product_of_scalars(plan, ops, g.diags, g.diags.back()), lim.total / NORM_MIN))
+                move_scalars(plan, ops, g.diags, g.diags.back(), &z2);
+            for (size_t k = 0; k + 1 < g.rots.size(); k += 2) move_scalars(plan, ops, {g.rots[k]}, g.rots[k + 1], &z2);
         }
         // reverse sweeps: both states carry the scalars taken out so far, so a
         // probe's sum carries their squared magnitude

@@ -427,3 +427,32 @@ def test_bound_coefficients_in_shared_memory(precision, layers):
     assert True in seen
     if layers == 12 and size == 8:
         assert False in seen
+
+
+@pytest.mark.parametrize("adjoint", [False, True])
+@pytest.mark.parametrize("sigma", [1e-1, 1e-3])
+def test_kernels_near_pi_have_two_forms_at_most(adjoint, sigma):
+    """A pass's code depends on which of its rotations are in unit form; over
+    the steps of a training near 0 and pi that is one of two patterns a pass,
+    so that steps do not keep meeting kernels that were not compiled yet."""
+    n, rng = 18, np.random.default_rng(3)
+    ops = [o for o in workloads.hea(n, 6, seed=0)[0] if o.name != "rz"]
+    rotations = [o for o in ops if o.slot >= 0]
+    base = rng.integers(0, 2, len(rotations)) * np.pi
+    lib, seen = nat.load(), {}
+    for step in range(12):
+        for k, (o, a) in enumerate(zip(rotations, base + rng.normal(0, sigma, len(rotations)))):
+            o.params, o.slot = (float(a),), k
+        if adjoint:
+            arr, pool = ir.pack(ops)
+            h = ctypes.c_void_p()
+            nat.check(lib.qfvm_plan_host_build_adjoint(n, 2, nat.vptr(arr), arr.size, nat.dptr(pool.view(np.float64)),
+                                                       pool.size, ctypes.byref(h)))
+        else:
+            h = plan_handle(n, ops, 2)
+        counts, shape = (ctypes.c_int64 * 4)(), (ctypes.c_int32 * 3)()
+        nat.check(lib.qfvm_plan_host_counts(h, counts, shape))
+        for i in range(counts[0]):
+            seen.setdefault(i, set()).add(pass_ptx(h, i, 2 if adjoint else 1))
+        lib.qfvm_plan_destroy(h)
+    assert max(len(s) for s in seen.values()) <= 2
