@@ -1148,7 +1148,9 @@ void fuse_single_qubit(std::vector<GOp>* gops) {
 }
 
 void unnormalize_hadamards(std::vector<GOp>* gops) {
-    constexpr int MAX_PENDING = 256;  // keeps |amplitudes| below 2^128 between absorptions
+    // |amplitudes| stay below 2^64 between absorptions: with the 2^48 of
+    // normalize_passes (NORM_ONE_STATE) on top, FP32 holds them
+    constexpr int MAX_PENDING = 128;
     std::vector<size_t> pending;
     int last = -1;
     for (size_t i = 0; i < gops->size(); ++i) {

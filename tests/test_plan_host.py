@@ -496,3 +496,26 @@ def test_sweep_probes_stay_in_single_precision(monkeypatch, precision, ansatz, n
     for v, s in zip(vals, plan["probe_slots"]):
         got[s] += v
     np.testing.assert_allclose(got, oracle.grad_adjoint(n, ops, [o.slot for o in ops], terms), atol=1e-8)
+
+
+@pytest.mark.parametrize("precision,T,R", [(1, 12, 4), (2, 12, 3)])
+def test_hadamards_and_unit_rotations_stay_in_single_precision(monkeypatch, precision, T, R):
+    """Hadamards without their 1/sqrt(2) (up to 128 before a gate takes their
+    scalar) while rotations near pi are in unit form (2^48 at most)."""
+    n, near = 14, np.pi - 2.0 ** -14
+    ops = [workloads.named("ry", (q,), (near,)) for q in (0, 1, 2)]
+    ops += [workloads.named("h", (q,)) for _ in range(125) for q in (5, 6)]
+    ops += [workloads.named("ry", (5,), (0.3,))] + [workloads.named("ry", (q,), (near,)) for q in (0, 1, 2)]
+    ops += [workloads.named("ry", (7,), (0.3,))]
+    plan = helpers.host_plan(n, ops, precision, T, R)
+    largest = [0.0]
+    inner = helpers.apply_global
+
+    def apply(psi, *args):
+        inner(psi, *args)
+        largest[0] = max(largest[0], float(np.abs(psi).max()))
+
+    monkeypatch.setattr(helpers, "apply_global", apply)
+    got = helpers.interpret(plan, oracle.zero_state(n))
+    assert largest[0] < 2.0 ** 113
+    assert np.abs(got - oracle.simulate(n, ops)).max() < 1e-13
