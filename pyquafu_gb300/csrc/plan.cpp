@@ -1219,22 +1219,38 @@ constexpr double NORM_MIN = 0x1p-24;
 
 bool uncontrolled(const KOp& o) { return o.cthr == 0 && o.creg == 0; }
 
+using cl = std::complex<long double>;
+
+// 1 / |(1, t)|, the scalar that leaves a rotation with off-diagonal entries t
+// and -t (or -it and -it) unitary whatever t was rounded to; c itself where
+// the gate is not a rotation
+long double rotation_scalar(double c, double s) {
+    if (!(std::fabs(c * c + s * s - 1.0) < 0x1p-48)) return c;
+    const long double t = s / c;
+    return std::copysign(1.0L / std::sqrt(1.0L + t * t), static_cast<long double>(c));
+}
+
 // a rotation with equal diagonal entries, or a two-valued phase of register
-// bits: the scalar that makes its first diagonal entry 1
-bool scalar_of(const KOp& o, const double* c, cd* f) {
+// bits: the scalar that makes its first diagonal entry 1.  Products of them are
+// formed in long double: rounded one by one to double they were the largest
+// error of a FP64 plan beside the amplitudes' own roundings.
+bool scalar_of(const KOp& o, const double* c, cl* f) {
     if (!uncontrolled(o)) return false;
-    if (o.kind == K_REAL) {
-        if (c[0] != c[3]) return false;
-        *f = cd(c[0], 0.0);
-    } else if (o.kind == K_RX) {
-        *f = cd(c[0], 0.0);
+    double size = 0.0;
+    if (o.kind == K_REAL || o.kind == K_RX) {
+        if (o.kind == K_REAL && c[0] != c[3]) return false;
+        size = std::fabs(c[0]);
     } else if (o.kind == K_DIAG) {
         if (o.flags & (F_D0_ONE | F_D1_SPEC | F_UNIFORM | F_TPAR)) return false;
-        *f = cd(c[0], c[1]);
+        size = std::hypot(c[0], c[1]);
     } else {
         return false;
     }
-    return std::abs(*f) >= NORM_MIN && std::abs(*f) <= 1.0 / NORM_MIN;
+    if (!(size >= NORM_MIN && size <= 1.0 / NORM_MIN)) return false;
+    if (o.kind == K_RX) *f = rotation_scalar(c[0], c[1]);
+    else if (o.kind == K_REAL) *f = c[1] == -c[2] ? rotation_scalar(c[0], c[2]) : c[0];
+    else *f = cl(c[0], c[1]);
+    return true;
 }
 
 // number of (complex) coefficients a scalar multiplies into at no cost: the
@@ -1249,35 +1265,35 @@ int free_scalar_coefs(const KOp& o, bool probes) {
     return 0;
 }
 
-void scale_complex(double* c, int n, cd z) {
+void scale_complex(double* c, int n, cl z) {
     for (int i = 0; i < n; ++i) {
-        const cd v = cd(c[2 * i], c[2 * i + 1]) * z;
-        c[2 * i] = v.real();
-        c[2 * i + 1] = v.imag();
+        const cl v = cl(c[2 * i], c[2 * i + 1]) * z;
+        c[2 * i] = static_cast<double>(v.real());
+        c[2 * i + 1] = static_cast<double>(v.imag());
     }
 }
 
 // ops: a pass's operations in order; `from`: some of them with a scalar
-cd product_of_scalars(HostPlan* plan, const std::vector<int>& ops, const std::vector<size_t>& from, size_t keeper) {
-    cd total(1.0, 0.0), f;
+cl product_of_scalars(HostPlan* plan, const std::vector<int>& ops, const std::vector<size_t>& from, size_t keeper) {
+    cl total(1.0L, 0.0L), f;
     for (size_t i : from)
         if (i != keeper && scalar_of(plan->ops[ops[i]], plan->coef.data() + plan->ops[ops[i]].coef, &f)) total *= f;
     return total;
 }
 
-bool in_range(cd z, double least) { return std::abs(z) >= least && std::abs(z) <= 1.0 / least; }
+bool in_range(cl z, double least) { return std::abs(z) >= least && std::abs(z) <= 1.0 / least; }
 
 // Takes the scalars of `from` (but the keeper's) out and multiplies the keeper
 // by their product; z2: the factors on |state|^2 from each operation on.
 void move_scalars(HostPlan* plan, const std::vector<int>& ops, const std::vector<size_t>& from, size_t keeper,
                   std::vector<double>* z2) {
-    const cd total = product_of_scalars(plan, ops, from, keeper);
-    cd f;
+    const cl total = product_of_scalars(plan, ops, from, keeper);
+    cl f;
     for (size_t i : from) {
         KOp& o = plan->ops[ops[i]];
         double* c = plan->coef.data() + o.coef;
         if (i == keeper || !scalar_of(o, c, &f)) continue;
-        (*z2)[i] /= std::norm(f);
+        (*z2)[i] /= static_cast<double>(std::norm(f));
         if (o.kind == K_REAL) {
             c[1] /= c[0];
             c[2] /= c[0];
@@ -1288,23 +1304,23 @@ void move_scalars(HostPlan* plan, const std::vector<int>& ops, const std::vector
             c[0] = 1.0;
             o.special = SP_UNIT;
         } else {
-            const cd d1 = cd(c[2], c[3]) / f;
+            const cl d1 = cl(c[2], c[3]) / f;
             c[0] = 1.0;
             c[1] = 0.0;
-            c[2] = d1.real();
-            c[3] = d1.imag();
+            c[2] = static_cast<double>(d1.real());
+            c[3] = static_cast<double>(d1.imag());
             o.flags |= F_D0_ONE;
         }
     }
-    if (total == cd(1.0, 0.0)) return;
+    if (total == cl(1.0L, 0.0L)) return;
     const KOp& o = plan->ops[ops[keeper]];
     double* c = plan->coef.data() + o.coef;
     if (o.kind == K_REAL || o.kind == K_RX) {
-        for (int i = 0; i < (o.kind == K_REAL ? 4 : 2); ++i) c[i] *= total.real();
+        for (int i = 0; i < (o.kind == K_REAL ? 4 : 2); ++i) c[i] = static_cast<double>(c[i] * total.real());
     } else {
         scale_complex(c, o.kind == K_DIAG ? 2 : free_scalar_coefs(o, false), total);
     }
-    (*z2)[keeper] *= std::norm(total);
+    (*z2)[keeper] *= static_cast<double>(std::norm(total));
 }
 
 }  // namespace
@@ -1329,7 +1345,7 @@ void normalize_passes(HostPlan* plan) {
         bool within = true;
         for (size_t i0 = 0, i1 = 0; i0 < ops.size(); i0 = i1) {
             Group g{{}, {}, ops.size()};
-            cd f;
+            cl f;
             for (i1 = i0; i1 < ops.size() && static_cast<int>(g.diags.size() + g.rots.size()) <= lim.count; ++i1) {
                 const KOp& o = plan->ops[ops[i1]];
                 if (free_scalar_coefs(o, pd.nprobe > 0)) g.keeper = i1;

@@ -519,3 +519,30 @@ def test_hadamards_and_unit_rotations_stay_in_single_precision(monkeypatch, prec
     got = helpers.interpret(plan, oracle.zero_state(n))
     assert largest[0] < 2.0 ** 113
     assert np.abs(got - oracle.simulate(n, ops)).max() < 1e-13
+
+
+def test_unit_rotations_keep_the_norm():
+    """The scalars of unit rotations go back as one product: what the plan's
+    rotations do to the norm is no further from 1 than what the gates do
+    rounded one by one (rms of 12 circuits, in long double)."""
+    n, plans, gates = 12, [], []
+    for seed in range(12):
+        rng = np.random.default_rng(seed)
+        ops = []
+        for _ in range(30):
+            ops += [workloads.named(["ry", "rx"][int(rng.integers(2))], (q,), (float(rng.uniform(0, 2 * np.pi)),))
+                    for q in range(n)]
+            ops += [workloads.named("cx", rng.choice(n, 2, replace=False), ncontrols=1) for _ in range(4)]
+        half = np.array([o.params[0] / 2 for o in ops if o.params])
+        c, s = np.cos(half).astype(np.longdouble), np.sin(half).astype(np.longdouble)
+        gates.append(np.log(c * c + s * s).sum())
+        plan = helpers.host_plan(n, ops, 0, 11, 4)
+        drift = np.longdouble(0)
+        for o in plan["ops"]:
+            m = plan["coef"][int(o["coef"]): int(o["coef"]) + 4].astype(np.longdouble)
+            if int(o["kind"]) == helpers.K_REAL:
+                drift += np.log(m[0] * m[3] - m[1] * m[2])
+            elif int(o["kind"]) == helpers.K_RX:
+                drift += np.log(m[0] * m[0] + m[1] * m[1])
+        plans.append(drift)
+    assert np.sqrt(np.mean(np.square(plans))) <= np.sqrt(np.mean(np.square(gates)))
