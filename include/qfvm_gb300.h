@@ -302,8 +302,10 @@ int qfvm_simulate_noise(int32_t num_qubits, const qfvm_op* ops, int64_t n_ops, c
  * qfvm_expect_statevec.
  *
  * A run takes the slot values of all groups back to back (group order, then
- * item-major) and writes expvals[item * n_obs + o] = <O_o> (FP64 sums) for all
- * groups back to back.  Mode 1 (batch created with QFVM_BATCH_GRADS) also
+ * item-major) and writes expvals[item * n_obs + o] = <psi|O_o|psi> (FP64 sums)
+ * for all groups back to back; a complex64 group whose gates are all unitary
+ * (matrix gates are looked at when the group is added) may divide it, and its
+ * gradients, by <psi|psi>, which then differs from 1 by rounding alone.  Mode 1 (batch created with QFVM_BATCH_GRADS) also
  * writes grads[item * n_slots + s] = d(sum_o w[item, o] <O_o>)/d value[s], by
  * the adjoint method, with weights w laid out like expvals (NULL: all 1).
  * Groups run concurrently on their own streams; the first run of a mode is

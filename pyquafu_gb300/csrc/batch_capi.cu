@@ -269,10 +269,11 @@ int add_group(qfvm_batch* b, int n, const qfvm_op* ops, int64_t n_ops, const dou
     const size_t b_ep = align256(static_cast<size_t>(chunks) * n_obs * 8);
     // complex64 states drift from unit norm with the rounding of their gates'
     // coefficients (about 3e-7 over 400 gates): their results are divided by
-    // <psi|psi>.  Not where one whole-state kernel runs every gate in the
+    // <psi|psi>.  Only where every gate is unitary: otherwise that norm is part
+    // of the result.  Not where one whole-state kernel runs every gate in the
     // interpreting arithmetic: the sums cost 3 to 5% of such a run (10 circuits
     // of 6 to 8 qubits: 279 us with them, 265 without).
-    const bool normed = storage == QFVM_C64 &&
+    const bool normed = storage == QFVM_C64 && known_unitary(ops, n_ops, matpool) &&
                         (g->fwd->hp.passes.empty() || g->fwd->hp.passes[0].type != PASS_SMALL);
     const size_t b_np = normed ? align256(static_cast<size_t>(chunks) * 8) : 0;
     const size_t b_inv = normed ? align256(static_cast<size_t>(n_items) * 8) : 0;

@@ -262,6 +262,9 @@ void simplify_plain(std::vector<GOp>* gops);
 // between their places and that point.  Entries that come out exactly 1,
 // -1, i or -i are coded so the kernels apply them without arithmetic.
 void merge_round_diagonals(HostPlan* plan);
+// Whether every gate of a classified op list is unitary (matrix gates to 1e-9;
+// false where a matrix on more than MAXK targets is not looked at).
+bool known_unitary(const qfvm_op* ops, int64_t n_ops, const double* matpool);
 // Plans without binds: inside every tile pass, uncontrolled rotations
 // [[c, -s], [s, c]] and [[c, -is], [-is, c]] become c * (1 on the diagonal)
 // and register-bit phases d0 * diag(1, d1 / d0); the scalars' product, which

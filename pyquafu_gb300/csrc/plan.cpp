@@ -1078,6 +1078,23 @@ void scale_coefs(GOp& g, int halves) {
 
 }  // namespace
 
+bool known_unitary(const qfvm_op* ops, int64_t n_ops, const double* matpool) {
+    constexpr double TOL = 1e-9;  // far below complex64's rounding
+    for (int64_t i = 0; i < n_ops; ++i) {
+        if (ops[i].kind != QFVM_OP_MATRIX) continue;  // the named gates are
+        const int64_t dim = ops[i].mat_dim;
+        if (dim > (1 << MAXK)) return false;
+        const cd* m = reinterpret_cast<const cd*>(matpool) + ops[i].mat_offset;
+        for (int64_t a = 0; a < dim; ++a)
+            for (int64_t b = a; b < dim; ++b) {  // columns a and b
+                cd s(a == b ? -1.0 : 0.0, 0.0);
+                for (int64_t r = 0; r < dim; ++r) s += std::conj(m[r * dim + a]) * m[r * dim + b];
+                if (!(std::abs(s) <= TOL)) return false;
+            }
+    }
+    return true;
+}
+
 namespace {
 
 uint64_t targets_of(const GOp& g) {

@@ -196,3 +196,24 @@ def test_bound_coefficient_ranges(precision, n, layers):
         e, ge = oracle_item(n, ops, vals[i], terms)
         assert abs(ev[0][i, 0] - e) < vtol
         np.testing.assert_allclose(g[0][i], ge, atol=gtol)
+
+
+@pytest.mark.parametrize("n", [8, 14])
+@pytest.mark.parametrize("precision,tol", [("c64", 1e-5), ("c128", 1e-12), ("c128_ds", 1e-12)])
+def test_non_unitary_gates_keep_their_norm(n, precision, tol):
+    """A group may hold matrix gates that are not unitary: its results are
+    <psi|O|psi> of that state in every arithmetic and at every size (the
+    whole-state kernel's and the tile passes')."""
+    ops = workloads.random_layers(n, 2, seed=n)
+    ops += [workloads.matrix_gate("damp", (0,), np.diag([1.0, 0.5])), ir.Op("ry", ir.OP_RY, (n - 1,), 0, (0.0,), slot=0),
+            workloads.matrix_gate("damp", (n - 1,), [[0.9, 0.1], [0.0, 0.6]])]
+    terms = [[(1.0, "Z", [0]), (0.3, "XX", [1, n - 1])], [(1.0, "Z", [n - 1])]]
+    vals = np.array([[0.4], [1.9]])
+    with BatchSession(precision) as bs:
+        bs.add_group(n, ops, terms, 2, 1)
+        ev = bs.run([vals])
+    for i in range(2):
+        psi = oracle.simulate(n, gradients.bind(ops, vals[i]))
+        assert np.linalg.norm(psi) < 0.95
+        ref = [sum(c * oracle.expect_pauli(psi, p, q) for c, p, q in o) for o in terms]
+        np.testing.assert_allclose(ev[0][i], ref, atol=tol)
