@@ -584,11 +584,12 @@ constexpr size_t PLAN_CHOICES = 32;
 std::mutex g_choices_mu;
 std::list<std::pair<std::string, Choices>> g_choices;  // most recent first
 
-std::string choices_key(int n, int T, int R, int cap, const std::vector<SchedOp>& ops) {
+std::string choices_key(int n, int eb, int T, int R, int cap, const std::vector<SchedOp>& ops) {
     std::string k;
     k.reserve(ops.size() * 36 + 16);
     auto put = [&](const auto& v) { k.append(reinterpret_cast<const char*>(&v), sizeof v); };
     put(n);
+    put(eb);  // the registers' padding (register_pad_order)
     put(T);
     put(R);
     put(cap);
@@ -717,7 +718,7 @@ bool build_plan(int n, int precision, const std::vector<GOp>& gops, int T, int R
     }
     const int cap = pass_op_cap(R, two_states, bound);
     const uint64_t low = (1ULL << L) - 1, every = n >= 64 ? ~0ULL : (1ULL << n) - 1;
-    std::string key = choices_key(n, T, R, cap, sops);
+    std::string key = choices_key(n, eb, T, R, cap, sops);
     Choices choices;
     const bool known = find_choices(key, &choices);
     size_t next_choice = 0;

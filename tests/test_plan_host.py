@@ -546,3 +546,20 @@ def test_unit_rotations_keep_the_norm():
                 drift += np.log(m[0] * m[0] + m[1] * m[1])
         plans.append(drift)
     assert np.sqrt(np.mean(np.square(plans))) <= np.sqrt(np.mean(np.square(gates)))
+
+
+@pytest.mark.parametrize("seed", [41, 42])
+def test_plans_do_not_depend_on_earlier_ones(seed):
+    """The sets kept for a structure are those of one amplitude size: complex64
+    and complex128 plans of one shape, in either order, and alone."""
+    n, first = 16, {}
+    for order in ((0, 1), (1, 0)):
+        ops = workloads.random_layers(n, 12, seed=seed, extras=True)
+        for k in range(order[0] * 40):  # pushes the kept sets of the first order out
+            helpers.host_plan(n, [workloads.named("h", (q,)) for q in range(1 + k % 8)] +
+                              [workloads.named("x", (k // 8,)), workloads.named("h", (k // 8,))], 0, 12, 4)
+        for precision in order:
+            plan = helpers.host_plan(n, ops, precision, 12, 4)
+            ref = first.setdefault(precision, plan)
+            for field in ("passes", "steps", "ops"):
+                assert np.array_equal(plan[field], ref[field]), (order, precision, field)
