@@ -574,15 +574,21 @@ uint64_t best_set(const std::vector<SchedOp>& ops, const std::vector<int>& todo,
 // The sets chosen for a circuit's passes and rounds, in order.  They depend on
 // the circuit's structure alone, and finding them costs milliseconds (30 qubits,
 // 1800 gates: 15 ms, then 1.6), so re-planning a structure at other angles looks them
-// up: the last PLAN_CHOICES structures of the process, keyed by every field
-// the search reads.
+// up: the last PLAN_CHOICES structures of the process, up to
+// PLAN_CHOICE_BYTES of keys and sets, keyed by every field the search reads.
 struct Choices {
     std::vector<uint64_t> sets;
 };
 constexpr size_t PLAN_CHOICES = 32;
+constexpr size_t PLAN_CHOICE_BYTES = 16 << 20;
 
 std::mutex g_choices_mu;
 std::list<std::pair<std::string, Choices>> g_choices;  // most recent first
+size_t g_choice_bytes = 0;
+
+size_t choice_bytes(const std::pair<std::string, Choices>& c) {
+    return c.first.capacity() + c.second.sets.capacity() * sizeof(uint64_t);
+}
 
 std::string choices_key(int n, int eb, int T, int R, int cap, const std::vector<SchedOp>& ops) {
     std::string k;
@@ -616,8 +622,14 @@ bool find_choices(const std::string& key, Choices* c) {
 
 void keep_choices(std::string key, Choices c) {
     std::lock_guard<std::mutex> lk(g_choices_mu);
+    for (const auto& kept : g_choices)
+        if (kept.first == key) return;  // another thread planned it meanwhile
     g_choices.emplace_front(std::move(key), std::move(c));
-    if (g_choices.size() > PLAN_CHOICES) g_choices.pop_back();
+    g_choice_bytes += choice_bytes(g_choices.front());
+    while (!g_choices.empty() && (g_choices.size() > PLAN_CHOICES || g_choice_bytes > PLAN_CHOICE_BYTES)) {
+        g_choice_bytes -= choice_bytes(g_choices.back());
+        g_choices.pop_back();
+    }
 }
 
 // Operations of one tile pass at most.  Fewer and larger passes are faster up

@@ -563,3 +563,32 @@ def test_plans_do_not_depend_on_earlier_ones(seed):
             ref = first.setdefault(precision, plan)
             for field in ("passes", "steps", "ops"):
                 assert np.array_equal(plan[field], ref[field]), (order, precision, field)
+
+
+def test_kept_sets_are_bounded_in_bytes():
+    """Structures of 100 K gates each (3.7 MB of key): what stays on the heap
+    after planning ten of them is below the 16 MiB that are kept, and a margin."""
+    import ctypes
+
+    class Info(ctypes.Structure):
+        _fields_ = [(k, ctypes.c_size_t) for k in ("arena", "ordblks", "smblks", "hblks", "hblkhd", "usmblks", "fsmblks",
+                                                   "uordblks", "fordblks", "keepcost")]
+
+    libc = ctypes.CDLL(None)
+    if not hasattr(libc, "mallinfo2"):
+        pytest.skip("no mallinfo2")
+    libc.mallinfo2.restype = Info
+
+    def used():
+        m = libc.mallinfo2()
+        return m.uordblks + m.hblkhd
+
+    def plan(k):
+        helpers.host_plan(12, [workloads.named("ry", (q % 12,), (0.3,)) for q in range(k, k + 12)] * 8400 +
+                          [workloads.named("h", (k,))], 0, 11, 4)
+
+    plan(0)
+    before = used()
+    for k in range(1, 11):
+        plan(k)
+    assert used() - before < 20 << 20
