@@ -367,6 +367,11 @@ int qfvm_plan_host_binds(const qfvm_plan* plan, int64_t* count, int32_t* records
 /* Parameter slot of each probe of an adjoint plan, in probe-id order. */
 int qfvm_plan_host_probe_slots(const qfvm_plan* plan, int32_t* slots);
 int qfvm_plan_host_counts(const qfvm_plan* plan, int64_t counts[4], int32_t shape[3]);
+/* Shots that a trajectory run (qfvm_simulate_shots, qfvm_simulate_noise) holds
+ * on the device at once with free_bytes free, item_bytes a shot (its state
+ * included), and whether it also holds the state that they start from. */
+int qfvm_host_items_memory(int64_t free_bytes, int32_t num_qubits, int64_t item_bytes, int64_t shots, int64_t* chunk,
+                           int32_t* shared);
 int qfvm_plan_host_copy(const qfvm_plan* plan, void* passes, void* steps, void* kops, double* coef);
 
 /* ---------------------------------------------------------------------------

@@ -107,6 +107,8 @@ PROTOTYPES = {
     "qfvm_plan_host_build": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int32, c_vp, ctypes.c_int64, c_dp,
                                             ctypes.c_int64, ctypes.c_int32, ctypes.c_int32, ctypes.POINTER(c_vp)]),
     "qfvm_plan_host_counts": (ctypes.c_int, [c_vp, ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int32)]),
+    "qfvm_host_items_memory": (ctypes.c_int, [ctypes.c_int64, ctypes.c_int32, ctypes.c_int64, ctypes.c_int64,
+                                              ctypes.POINTER(ctypes.c_int64), c_i32p]),
     "qfvm_plan_host_build_adjoint": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int32, c_vp, ctypes.c_int64, c_dp,
                                                     ctypes.c_int64, ctypes.POINTER(c_vp)]),
     "qfvm_plan_host_build_batched": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int32, c_vp, ctypes.c_int64, c_dp,

@@ -133,6 +133,16 @@ int make_plan(int n, int precision, const qfvm_op* ops, int64_t n_ops, const dou
 int make_plan_gops(int n, int precision, const std::vector<qsv::GOp>& gops, int T, int R, qfvm_plan** out,
                    bool merge_diagonals = false);
 void free_plan(qfvm_plan* p);
+// Shots (items) of a trajectory run that are on the device at once, given the
+// free memory, a state's bytes and an item's (its state among them): about half
+// of the free memory, the state that they start from counted.  `shared`: that
+// state is held and copied to the items.  A run of one shot, and one whose
+// memory holds one item but not that state as well, prepares each item in place.
+struct ItemsMemory {
+    int64_t chunk;
+    bool shared;
+};
+ItemsMemory items_memory(size_t free_bytes, size_t state_bytes, size_t item_bytes, int64_t shots);
 // Every pass of a plan over `items` states back to back (shared coefficients;
 // active = optional per-item write-back mask).
 int run_plan_items(qfvm_plan* p, void* state, int items, const uint8_t* active, cudaStream_t st);

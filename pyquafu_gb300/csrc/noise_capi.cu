@@ -141,10 +141,8 @@ int qfvm_simulate_noise(int32_t num_qubits, const qfvm_op* ops, int64_t n_ops, c
     cudaMemGetInfo(&free_b, &total_b);
     const size_t per_item = (sizeof(double2) << n) + 8u * ndraws + 8u * bpi * (MAX_CHANNEL_OPS + 1) + 64 + 16 +
                             8u * static_cast<size_t>(n_terms) * (epi + 1);
-    int64_t chunk = static_cast<int64_t>((free_b / 2) / per_item);
-    if (chunk < 1) chunk = 1;
-    if (chunk > shots) chunk = shots;
-    if (chunk > (1 << 20)) chunk = 1 << 20;
+    const ItemsMemory mem = items_memory(free_b, sizeof(double2) << n, per_item, shots);
+    const int64_t chunk = mem.chunk;
 
     cudaStream_t st = nullptr;
     DevBuf dstate, dpsi0, duni, dscratch, dterms;
@@ -175,18 +173,21 @@ int qfvm_simulate_noise(int32_t num_qubits, const qfvm_op* ops, int64_t n_ops, c
     } while (0)
     NZ_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream");
     NZ_TRY(dstate.ensure(static_cast<size_t>(chunk) * N * sizeof(double2)));
-    // the shots share one state up to the first channel: prepared once, then copied
-    NZ_TRY(dpsi0.ensure(N * sizeof(double2)));
-    if (psi_in)
-        NZ_CUDA(cudaMemcpyAsync(dpsi0.p, psi_in, N * sizeof(double2), cudaMemcpyHostToDevice, st), "input upload");
-    else
-        NZ_CUDA(launch_zero_items(QFVM_C128, dpsi0.p, n, 1, st), "initial state");
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    size_t first = 0;
-    if (!segs.empty() && segs[0].type == 0) {
-        NZ_TRY(run_plan_items(segs[0].plan, dpsi0.p, 1, nullptr, st));
-        first = 1;
-    }
+    // the shots share one state up to the first channel: prepared once, then
+    // copied, or (one shot, or no room for it) prepared in the shot's own
+    if (mem.shared) NZ_TRY(dpsi0.ensure(N * sizeof(double2)));
+    void* const prep = mem.shared ? dpsi0.p : dstate.p;
+    auto prepare_start = [&]() -> int {
+        if (psi_in)
+            QSV_CUDA(cudaMemcpyAsync(prep, psi_in, N * sizeof(double2), cudaMemcpyHostToDevice, st), "input upload");
+        else
+            QSV_CUDA(launch_zero_items(QFVM_C128, prep, n, 1, st), "initial state");
+        g_launches.fetch_add(1, std::memory_order_relaxed);
+        if (!segs.empty() && segs[0].type == 0) return run_plan_items(segs[0].plan, prep, 1, nullptr, st);
+        return QFVM_OK;
+    };
+    const size_t first = !segs.empty() && segs[0].type == 0 ? 1 : 0;
+    if (mem.shared) NZ_TRY(prepare_start());
     NZ_TRY(duni.ensure(static_cast<size_t>(chunk) * ndraws * 8));
     // scratch: channel data, channel norms, per-item matrices, samples, expectation chunks and values
     const size_t b_cd = align256(std::max<size_t>(cdata.size(), 1) * 8);
@@ -238,9 +239,14 @@ int qfvm_simulate_noise(int32_t num_qubits, const qfvm_op* ops, int64_t n_ops, c
         NZ_CUDA(cudaMemcpyAsync(duni.p, uniforms + c0 * ndraws, static_cast<size_t>(items) * ndraws * 8,
                                 cudaMemcpyHostToDevice, st),
                 "uniform upload");
-        NZ_CUDA(launch_items_copy(dstate.p, n, items, dpsi0.p, st), "initial states");
+        if (mem.shared) {
+            NZ_CUDA(launch_items_copy(dstate.p, n, items, dpsi0.p, st), "initial states");
+            g_launches.fetch_add(1, std::memory_order_relaxed);
+        } else {
+            NZ_TRY(prepare_start());
+        }
         NZ_CUDA(launch_fill_ones(dscale, items, st), "initial scales");
-        g_launches.fetch_add(2, std::memory_order_relaxed);
+        g_launches.fetch_add(1, std::memory_order_relaxed);
         for (size_t si = first; si < segs.size(); ++si) {
             const NoiseSegment& sg = segs[si];
             if (sg.type == 0) {

@@ -117,6 +117,14 @@ int parse_program(int n, int ncb, const qfvm_op* ops, int64_t n_ops, const doubl
 
 namespace qsv_capi {
 
+ItemsMemory items_memory(size_t free_bytes, size_t state_bytes, size_t item_bytes, int64_t shots) {
+    const size_t half = free_bytes / 2;
+    int64_t chunk = half > state_bytes ? static_cast<int64_t>((half - state_bytes) / item_bytes) : 0;
+    chunk = std::min<int64_t>({std::max<int64_t>(chunk, 1), shots, 1 << 20});
+    constexpr size_t MARGIN = 64 << 20;  // allocation granularity, the other small buffers
+    return {chunk, shots > 1 && free_bytes >= state_bytes + static_cast<size_t>(chunk) * item_bytes + MARGIN};
+}
+
 // Every pass of a plan over `items` states (shared coefficient pool).
 int run_plan_items(qfvm_plan* p, void* state, int items, const uint8_t* active, cudaStream_t st) {
     if (active) p->chain_ok = false;  // inactive items keep their FP64 state: no float pairs between passes
@@ -145,6 +153,17 @@ int run_plan_items(qfvm_plan* p, void* state, int items, const uint8_t* active, 
 }  // namespace qsv_capi
 
 extern "C" {
+
+int qfvm_host_items_memory(int64_t free_bytes, int32_t num_qubits, int64_t item_bytes, int64_t shots, int64_t* chunk,
+                           int32_t* shared) {
+    if (free_bytes < 0 || num_qubits < 1 || num_qubits > QFVM_MAX_QUBITS || item_bytes < 1 || shots < 1 || !chunk || !shared)
+        return fail(QFVM_ERR_INVALID, "bad trajectory sizes");
+    const ItemsMemory m = items_memory(static_cast<size_t>(free_bytes), sizeof(double2) << num_qubits,
+                                       static_cast<size_t>(item_bytes), shots);
+    *chunk = m.chunk;
+    *shared = m.shared ? 1 : 0;
+    return QFVM_OK;
+}
 
 int qfvm_simulate_shots(int32_t num_qubits, int32_t num_cbits, const qfvm_op* ops, int64_t n_ops,
                         const double* matpool, int64_t matpool_len, const double* psi_in, int64_t shots,
@@ -179,15 +198,12 @@ int qfvm_simulate_shots(int32_t num_qubits, int32_t num_cbits, const qfvm_op* op
                 for (int j = 0; j < sg.ms.k; ++j) measured.insert(sg.ms.cb[j]);
         }
 
-    // chunk of shots resident at once: at most about half of the free memory
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
     const size_t per_item = (sizeof(double2) << n) + static_cast<size_t>(ncb) + 64 +
                             static_cast<size_t>(outcome_blocks_per_item(n, 1)) * (8u << kmax) + 8u * ndraws;
-    int64_t chunk = static_cast<int64_t>((free_b / 2) / per_item);
-    if (chunk < 1) chunk = 1;
-    if (chunk > shots) chunk = shots;
-    if (chunk > (1 << 20)) chunk = 1 << 20;
+    const ItemsMemory mem = items_memory(free_b, sizeof(double2) << n, per_item, shots);
+    const int64_t chunk = mem.chunk;
 
     cudaStream_t st = nullptr;
     DevBuf dstate, dpsi0, duni, dcreg, dscratch;
@@ -220,18 +236,21 @@ int qfvm_simulate_shots(int32_t num_qubits, int32_t num_cbits, const qfvm_op* op
     const size_t N = 1ULL << n;
     SHOT_TRY(dstate.ensure(static_cast<size_t>(chunk) * N * sizeof(double2)));
     // Every shot starts from one state, and it stays one up to the first
-    // measure, reset or cif: that state is prepared once and copied to the shots.
-    SHOT_TRY(dpsi0.ensure(N * sizeof(double2)));
-    if (psi_in)
-        SHOT_CUDA(cudaMemcpyAsync(dpsi0.p, psi_in, N * sizeof(double2), cudaMemcpyHostToDevice, st), "input upload");
-    else
-        SHOT_CUDA(launch_zero_items(QFVM_C128, dpsi0.p, n, 1, st), "initial state");
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    size_t first = 0;
-    if (!segs.empty() && segs[0].type == 0) {
-        SHOT_TRY(run_plan_items(segs[0].plan, dpsi0.p, 1, nullptr, st));
-        first = 1;
-    }
+    // measure, reset or cif: that state is prepared once and copied to the
+    // shots, or (one shot, or no room for it) prepared in the shot's own.
+    if (mem.shared) SHOT_TRY(dpsi0.ensure(N * sizeof(double2)));
+    void* const prep = mem.shared ? dpsi0.p : dstate.p;
+    auto prepare_start = [&]() -> int {
+        if (psi_in)
+            QSV_CUDA(cudaMemcpyAsync(prep, psi_in, N * sizeof(double2), cudaMemcpyHostToDevice, st), "input upload");
+        else
+            QSV_CUDA(launch_zero_items(QFVM_C128, prep, n, 1, st), "initial state");
+        g_launches.fetch_add(1, std::memory_order_relaxed);
+        if (!segs.empty() && segs[0].type == 0) return run_plan_items(segs[0].plan, prep, 1, nullptr, st);
+        return QFVM_OK;
+    };
+    const size_t first = !segs.empty() && segs[0].type == 0 ? 1 : 0;
+    if (mem.shared) SHOT_TRY(prepare_start());
     SHOT_TRY(duni.ensure(static_cast<size_t>(chunk) * std::max(ndraws, 1) * 8));
     SHOT_TRY(dcreg.ensure(static_cast<size_t>(chunk) * ncb));
     const size_t b_part = align256(static_cast<size_t>(chunk) * outcome_blocks_per_item(n, 1) * (8u << kmax));
@@ -254,8 +273,10 @@ int qfvm_simulate_shots(int32_t num_qubits, int32_t num_cbits, const qfvm_op* op
         const bool last = c0 + items >= shots;
         // a measure or reset of the shared state reads it from dpsi0 and writes
         // the collapsed states; anything else starts from copies
-        bool shared = first < segs.size() && segs[first].type == 1;
-        if (!shared) {
+        bool shared = mem.shared && first < segs.size() && segs[first].type == 1;
+        if (!mem.shared) {
+            SHOT_TRY(prepare_start());
+        } else if (!shared) {
             SHOT_CUDA(launch_items_copy(dstate.p, n, items, dpsi0.p, st), "initial states");
             g_launches.fetch_add(1, std::memory_order_relaxed);
         }

@@ -105,3 +105,30 @@ def test_shared_first_state_and_unread_last_states(n, start, end, shots):
     ref_out, ref_final = oracle.simulate_shots(n, ops, ncb, uni, psi)
     assert out.tolist() == ref_out
     assert np.max(np.abs(final - ref_final)) < 1e-12
+
+
+def test_one_shot_at_a_time_without_room_for_the_shared_state():
+    """Memory for one shot but not for the state that the shots start from:
+    every shot is prepared in its own state, from |0...0> and from an input."""
+    torch = pytest.importorskip("torch")
+    n, ncb, shots = 24, 2, 3
+    ops = workloads.random_layers(n, 1, seed=n)
+    ops.append(ir.Op("measure", ir.OP_MEASURE, qbits=[n - 1, 0], cbits=[0, 1]))
+    ops += [named("h", (0,)), ir.Op("measure", ir.OP_MEASURE, qbits=[0], cbits=[1])]
+    ref = {}
+    fill = None
+    for full in (False, True):
+        if full:
+            torch.cuda.synchronize()
+            free, _ = torch.cuda.mem_get_info()
+            fill = torch.empty(free - (16 << n) - (160 << 20), dtype=torch.uint8, device="cuda")
+        for psi in (np.zeros(0, dtype=np.complex128), helpers.random_state(n, 4)):
+            qfvm.set_seed(23)
+            out, final = qfvm._shots(n, ncb, ops, psi, shots)
+            if not full:
+                ref[psi.size] = (out.tolist(), final)
+            else:
+                assert out.tolist() == ref[psi.size][0]
+                assert np.array_equal(final, ref[psi.size][1])
+    del fill
+    torch.cuda.empty_cache()

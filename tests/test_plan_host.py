@@ -592,3 +592,26 @@ def test_kept_sets_are_bounded_in_bytes():
     for k in range(1, 11):
         plan(k)
     assert used() - before < 20 << 20
+
+
+@pytest.mark.parametrize("n,shots", [(12, 4096), (24, 10), (29, 1), (29, 3), (30, 1), (30, 100)])
+def test_trajectory_memory(n, shots):
+    """What a trajectory run holds: half of the free memory where more than one
+    shot fits with the state that they start from, that state only where it
+    fits and is used more than once, and never more than one shot's where that
+    is all there is room for."""
+    import ctypes
+
+    from pyquafu_gb300 import _native as nat
+
+    state, item = 16 << n, (16 << n) + 5000
+    for free in (item + 1000, 2 * state + 4000, 2 * item + (65 << 20), 4 * item, 284 << 30):
+        chunk, shared = ctypes.c_int64(), np.zeros(1, np.int32)
+        nat.check(nat.load().qfvm_host_items_memory(free, n, item, shots, ctypes.byref(chunk), nat.i32ptr(shared)))
+        held = chunk.value * item + int(shared[0]) * state
+        assert 1 <= chunk.value <= shots
+        assert held <= (free if chunk.value == 1 else free // 2)
+        assert held == item or shots > 1
+        if free == 284 << 30:
+            assert shared[0] == (shots > 1)
+            assert chunk.value == shots or held + item > free // 2
