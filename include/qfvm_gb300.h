@@ -357,7 +357,7 @@ int qfvm_plan_host_build(int32_t num_qubits, int32_t precision, const qfvm_op* o
 int qfvm_plan_host_build_adjoint(int32_t num_qubits, int32_t precision, const qfvm_op* ops, int64_t n_ops,
                                  const double* matpool, int64_t matpool_len, qfvm_plan** out);
 /* The forward plan (adjoint == 0) or reverse sweep (adjoint != 0) that a
- * batch group runs, host only: value-dependent fast paths of slotted gates are
+ * batch group of many items runs, host only: value-dependent fast paths of slotted gates are
  * dropped and the pool blocks a run rewrites per item are recorded. */
 int qfvm_plan_host_build_batched(int32_t num_qubits, int32_t precision, const qfvm_op* ops, int64_t n_ops,
                                  const double* matpool, int64_t matpool_len, int32_t adjoint, qfvm_plan** out);

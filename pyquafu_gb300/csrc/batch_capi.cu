@@ -171,7 +171,7 @@ int add_group(qfvm_batch* b, int n, const qfvm_op* ops, int64_t n_ops, const dou
         cudaEventCreateWithFlags(&g->done, cudaEventDisableTiming) != cudaSuccess)
         return bail(fail(QFVM_ERR_CUDA, "batch stream creation"));
     int fT = b->T, fR = b->R;
-    if (fT <= 0 && fR <= 0) batch_forward_shape(arith, n, &fT, &fR);
+    if (fT <= 0 && fR <= 0) batch_forward_shape(arith, n, n_items, &fT, &fR);
     int rc = make_plan_gops(n, arith, gops, fT, fR, &g->fwd);
     if (rc != QFVM_OK) return bail(rc);
     if (grads) {

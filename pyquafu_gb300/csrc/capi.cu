@@ -671,7 +671,7 @@ int qfvm_plan_host_build_batched(int32_t num_qubits, int32_t precision, const qf
         if (!build_adjoint_sweep(gops, &sweep, &err)) return fail(QFVM_ERR_INVALID, err);
         resolve_shape(precision, 1, num_qubits, &T, &R);
     } else {
-        batch_forward_shape(precision, num_qubits, &T, &R);
+        batch_forward_shape(precision, num_qubits, 1LL << 24, &T, &R);
     }
     qfvm_plan* p = new qfvm_plan();
     if (!build_plan(num_qubits, store_precision(precision), adjoint ? sweep : gops, T, R, &p->hp, &err)) {

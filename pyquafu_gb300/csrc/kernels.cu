@@ -186,25 +186,27 @@ __global__ void k_c64_to_c128(const float2* __restrict__ in, double2* __restrict
 // packed as T | R << 8; 0 means the built-in default.
 static std::atomic<int32_t> g_tuned[3][2][QFVM_MAX_QUBITS + 1];
 
-void resolve_shape(int arith, int kind, int n, int* T, int* R) {
+static bool tuned_shape(int arith, int kind, int n, int* T, int* R) {
     const int a = (arith == QFVM_C64) ? 1 : (arith == QFVM_C128_DS ? 2 : 0);
     const int32_t v = (n >= 0 && n <= QFVM_MAX_QUBITS && (kind == 0 || kind == 1))
                           ? g_tuned[a][kind][n].load(std::memory_order_relaxed)
                           : 0;
-    if (v) {
-        *T = v & 0xff;
-        *R = (v >> 8) & 0xff;
-        return;
-    }
+    if (!v) return false;
+    *T = v & 0xff;
+    *R = (v >> 8) & 0xff;
+    return true;
+}
+
+void resolve_shape(int arith, int kind, int n, int* T, int* R) {
+    if (tuned_shape(arith, kind, n, T, R)) return;
     if (kind == 1) adjoint_shape(arith, T, R);
     else default_shape(n, arith, T, R);
 }
 
-void batch_forward_shape(int arith, int n, int* T, int* R) {
-    resolve_shape(arith, 0, n, T, R);
-    int dT = 0, dR = 0;
-    default_shape(n, arith, &dT, &dR);
-    if (arith == QFVM_C64 && *T == dT && *R == dR) {
+void batch_forward_shape(int arith, int n, int64_t items, int* T, int* R) {
+    if (tuned_shape(arith, 0, n, T, R)) return;
+    default_shape(n, arith, T, R);
+    if (arith == QFVM_C64 && (n <= 14 || items < (152LL >> (n - 13)))) {
         *T = 12;
         *R = 4;
     }

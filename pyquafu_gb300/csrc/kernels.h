@@ -16,11 +16,14 @@ bool pass_shape_supported(int precision, int T, int R);
 // the autotuned one if set, else the built-in default.
 void resolve_shape(int arith, int kind, int n, int* T, int* R);
 bool set_tuned_shape(int arith, int kind, int n, int T, int R);
-// One-state shape of a batch group's forward plan (T = 0 asked for): as
-// resolve_shape, but complex64 groups default to (12, 4).  A hardware-efficient
-// ansatz puts most of its gates into the first pass, whose unrolled rounds at
-// five register qubits (22 K instructions) ran out of the instruction cache.
-void batch_forward_shape(int arith, int n, int* T, int* R);
+// One-state shape of a batch group's forward plan (T = 0 asked for): the tuned
+// one if set; else the default, but (12, 4) for complex64 groups of at most 14
+// qubits (6 layers, 2048 items: 12 qubits 334 us, 3.6 ms on the whole-state
+// kernel of a 13-qubit tile; 14 qubits 1185 us, 1236 at (13, 5)) and for those
+// that fill less than one tile of 13 qubits an SM (19 items of 15 qubits: 72 us,
+// 87 at (13, 5)).  Larger ones have fewer passes at (13, 5): 1024 items of 16
+// qubits, 12 layers, 3.99 ms, 4.36 at (12, 4).
+void batch_forward_shape(int arith, int n, int64_t items, int* T, int* R);
 bool pass_shape_c128(int T, int R);
 bool pass_shape_c64(int T, int R);
 bool pass_shape_ds(int T, int R);

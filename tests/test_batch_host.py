@@ -8,6 +8,7 @@ import pytest
 
 import helpers
 import oracle
+from pyquafu_gb300 import _native as nat
 from pyquafu_gb300 import gradients, ir, workloads
 
 named = workloads.named
@@ -149,3 +150,27 @@ def test_unbindable_slot_is_rejected():
     ops = [ir.Op("u", ir.OP_MATRIX, (0,), 0, (0.3,), matrix=m, slot=0)]
     with pytest.raises(nat.QfvmError, match="per-item parameter"):
         helpers.host_plan(2, ops, batched=True)
+
+
+def test_forward_shape_rule():
+    """Forward plans of complex64 groups: the tuned shape whatever it is, also
+    where it is the built-in one, else (12, 4) up to 14 qubits and the built-in
+    shape above."""
+    lib = nat.load()
+    ops, _ = workloads.hea(16, 2, seed=1, encode=np.zeros(16))
+
+    def shape(n):
+        gates = [o for o in ops if max(o.qubits) < n]
+        plan = helpers.host_plan(n, gates, nat.QFVM_C64, batched=True)
+        return plan["T"], plan["R"]
+
+    for n in (12, 13, 14):
+        assert shape(n) == (12, 4)
+    assert shape(15) == shape(16) == (13, 5)
+    for tuned in ((13, 5), (12, 5)):
+        for n in (13, 14, 16):
+            nat.check(lib.qfvm_set_tuned_shape(nat.QFVM_C64, 0, n, *tuned))
+            try:
+                assert shape(n) == tuned
+            finally:
+                nat.check(lib.qfvm_set_tuned_shape(nat.QFVM_C64, 0, n, 0, 0))
