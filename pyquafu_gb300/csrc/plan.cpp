@@ -633,17 +633,19 @@ void keep_choices(std::string key, Choices c) {
 }
 
 // Operations of one tile pass at most.  Fewer and larger passes are faster up
-// to where their unrolled code leaves the instruction cache: 27 qubits
-// complex64 (R = 5) 14.2 ms at 42 operations, 12.7 at 62, 12.9 without a limit;
-// the 24-qubit float-pair sweep (R = 3) 63.6 ms at 84, 63.3 at 125; batched
-// sweeps (R = 4) 23.3 ms at 42, 21.3 at 62, 19.1 without.  The limits below
-// are lower where the default plans of the 30-qubit and 24-qubit benchmark
-// circuits would otherwise have fewer than the 40 passes over which
-// tests/test_jit_host.py bounds the code size.
-int pass_op_cap(int R, bool two_states, bool bound) {
+// to where their unrolled code leaves the instruction cache, and that shows only
+// where a pass streams far more than the L2: complex64 (13, 5), depth 20 and 40,
+// 14 qubits 85 and 164 us at 45 operations, 62 and 110 without a limit; 20
+// qubits 137 and 251, 118 and 206; 25 qubits 2.05 and 3.84 ms, 1.80 and 3.49; 27
+// qubits 7.99 and 15.6 ms at 45, 7.51 and 14.2 at 62, 8.05 and 14.5 without.
+// Reverse sweeps do not depend on it (11 to 22 qubits: 2%), batched ones take
+// any number (23.3 ms at 42, 21.3 at 62, 19.1 without).  Above 26 qubits and for
+// sweeps the limits are lower than that asks for: tests/test_jit_host.py bounds
+// the code size over at least 40 passes of two benchmark circuits.
+int pass_op_cap(int n, int R, bool two_states, bool bound) {
     if (bound) return INT_MAX;
     if (two_states) return R <= 3 ? 84 : 62;
-    return R >= 5 ? 45 : INT_MAX;
+    return R >= 5 && n > 26 ? 45 : INT_MAX;
 }
 
 }  // namespace
@@ -728,7 +730,7 @@ bool build_plan(int n, int precision, const std::vector<GOp>& gops, int T, int R
         two_states |= g.kind == K_PROBE;
         bound |= g.bkind != 0 && g.slot >= 0 && g.kind != K_PROBE;
     }
-    const int cap = pass_op_cap(R, two_states, bound);
+    const int cap = pass_op_cap(n, R, two_states, bound);
     const uint64_t low = (1ULL << L) - 1, every = n >= 64 ? ~0ULL : (1ULL << n) - 1;
     std::string key = choices_key(n, eb, T, R, cap, sops);
     Choices choices;

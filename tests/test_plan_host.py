@@ -615,3 +615,12 @@ def test_trajectory_memory(n, shots):
         if free == 284 << 30:
             assert shared[0] == (shots > 1)
             assert chunk.value == shots or held + item > free // 2
+
+
+@pytest.mark.parametrize("precision,T", [(0, 11), (1, 13), (2, 12)])
+def test_small_states_have_few_passes(precision, T):
+    """A pass of a small state costs its latency, whatever it holds: a state of
+    one tile is one pass, one of two tiles few (20 layers)."""
+    for n, most in ((T, 1), (T + 1, 5)):
+        plan = helpers.host_plan(n, workloads.random_layers(n, 20, seed=3), precision)
+        assert plan["T"] == T and len(plan["passes"]) <= most
