@@ -1240,8 +1240,8 @@ namespace {
 // the limit, every second rotation of the pass its own: two patterns a pass
 // (gate by gate up to the limit, a circuit near pi met new patterns at almost
 // every step of a training).  At random angles a scalar is about 1/2 in the
-// geometric mean: 4e-8 of the gates are below NORM_MIN, 4e-6 and 6e-6 of the
-// groups beyond their limit.
+// geometric mean: 4e-8 of the gates are below NORM_MIN, 4e-6 (one state) and
+// 6e-6 (sweep) of the groups beyond their limit.
 struct NormLimits {
     int count;
     double total;
@@ -1251,22 +1251,61 @@ constexpr double NORM_MIN = 0x1p-24;
 
 bool uncontrolled(const KOp& o) { return o.cthr == 0 && o.creg == 0; }
 
-using cl = std::complex<long double>;
+// Numbers of 106 bits as the sum of two doubles (TwoSum, TwoProd with FMA;
+// Dekker 1971, Ogita, Rump and Oishi 2005).  (long double would do, but is
+// software on Arm: 24 qubits, 960 parameters, 2 ms a call.)
+struct Dd {
+    double h = 0.0, l = 0.0;
+};
+Dd two_sum(double a, double b) {
+    const double s = a + b, v = s - a;
+    return {s, (a - (s - v)) + (b - v)};
+}
+Dd two_prod(double a, double b) {
+    const double p = a * b;
+    return {p, std::fma(a, b, -p)};
+}
+Dd operator+(Dd a, Dd b) {
+    const Dd s = two_sum(a.h, b.h);
+    return two_sum(s.h, s.l + (a.l + b.l));
+}
+Dd operator-(Dd a) { return {-a.h, -a.l}; }
+Dd operator*(Dd a, Dd b) {
+    const Dd p = two_prod(a.h, b.h);
+    return two_sum(p.h, p.l + std::fma(a.h, b.l, a.l * b.h));
+}
+Dd operator/(Dd a, Dd b) {
+    const double q = a.h / b.h;
+    const Dd r = a + -(b * Dd{q, 0.0});
+    return two_sum(q, r.h / b.h);
+}
+
+struct Scalar {
+    Dd re, im;
+    double abs() const { return std::hypot(re.h, im.h); }
+    double norm() const { return re.h * re.h + im.h * im.h; }
+    bool one() const { return re.h == 1.0 && re.l == 0.0 && im.h == 0.0; }
+};
+Scalar operator*(const Scalar& a, const Scalar& b) {
+    if (a.im.h == 0.0 && b.im.h == 0.0) return {a.re * b.re, {}};
+    return {a.re * b.re + -(a.im * b.im), a.re * b.im + a.im * b.re};
+}
 
 // 1 / |(1, t)|, the scalar that leaves a rotation with off-diagonal entries t
-// and -t (or -it and -it) unitary whatever t was rounded to; c itself where
-// the gate is not a rotation
-long double rotation_scalar(double c, double s) {
-    if (!(std::fabs(c * c + s * s - 1.0) < 0x1p-48)) return c;
-    const long double t = s / c;
-    return std::copysign(1.0L / std::sqrt(1.0L + t * t), static_cast<long double>(c));
+// and -t (or -it and -it) unitary whatever t was rounded to (one Newton step
+// from c); c itself where the gate is not a rotation
+Dd rotation_scalar(double c, double s) {
+    if (!(std::fabs(c * c + s * s - 1.0) < 0x1p-48)) return {c, 0.0};
+    const Dd ct = two_prod(c, s / c);
+    const Dd r = Dd{1.0, 0.0} + -(two_prod(c, c) + ct * ct);
+    return two_sum(c, 0.5 * c * r.h);
 }
 
 // a rotation with equal diagonal entries, or a two-valued phase of register
-// bits: the scalar that makes its first diagonal entry 1.  Products of them are
-// formed in long double: rounded one by one to double they were the largest
-// error of a FP64 plan beside the amplitudes' own roundings.
-bool scalar_of(const KOp& o, const double* c, cl* f) {
+// bits: the scalar that makes its first diagonal entry 1.  Rounded to double
+// one product after the other, they were the largest error of an FP64 plan
+// beside the amplitudes' own roundings.
+bool scalar_of(const KOp& o, const double* c, Scalar* f) {
     if (!uncontrolled(o)) return false;
     double size = 0.0;
     if (o.kind == K_REAL || o.kind == K_RX) {
@@ -1279,9 +1318,10 @@ bool scalar_of(const KOp& o, const double* c, cl* f) {
         return false;
     }
     if (!(size >= NORM_MIN && size <= 1.0 / NORM_MIN)) return false;
-    if (o.kind == K_RX) *f = rotation_scalar(c[0], c[1]);
-    else if (o.kind == K_REAL) *f = c[1] == -c[2] ? rotation_scalar(c[0], c[2]) : c[0];
-    else *f = cl(c[0], c[1]);
+    *f = Scalar{};
+    if (o.kind == K_RX) f->re = rotation_scalar(c[0], c[1]);
+    else if (o.kind == K_REAL) f->re = c[1] == -c[2] ? rotation_scalar(c[0], c[2]) : Dd{c[0], 0.0};
+    else *f = Scalar{{c[0], 0.0}, {c[1], 0.0}};
     return true;
 }
 
@@ -1297,35 +1337,33 @@ int free_scalar_coefs(const KOp& o, bool probes) {
     return 0;
 }
 
-void scale_complex(double* c, int n, cl z) {
-    for (int i = 0; i < n; ++i) {
-        const cl v = cl(c[2 * i], c[2 * i + 1]) * z;
-        c[2 * i] = static_cast<double>(v.real());
-        c[2 * i + 1] = static_cast<double>(v.imag());
-    }
-}
+// A pass's operations in order, with their scalars.
+struct ScalarOp {
+    KOp* o;
+    double* c;
+    bool has;
+    Scalar f;
+    double z2;  // factor on |state|^2 from this operation on
+};
 
-// ops: a pass's operations in order; `from`: some of them with a scalar
-cl product_of_scalars(HostPlan* plan, const std::vector<int>& ops, const std::vector<size_t>& from, size_t keeper) {
-    cl total(1.0L, 0.0L), f;
+Scalar product_of_scalars(const std::vector<ScalarOp>& ops, const std::vector<size_t>& from, size_t keeper) {
+    Scalar total{{1.0, 0.0}, {}};
     for (size_t i : from)
-        if (i != keeper && scalar_of(plan->ops[ops[i]], plan->coef.data() + plan->ops[ops[i]].coef, &f)) total *= f;
+        if (i != keeper) total = total * ops[i].f;
     return total;
 }
 
-bool in_range(cl z, double least) { return std::abs(z) >= least && std::abs(z) <= 1.0 / least; }
+bool in_range(const Scalar& z, double least) { return z.abs() >= least && z.abs() <= 1.0 / least; }
 
 // Takes the scalars of `from` (but the keeper's) out and multiplies the keeper
-// by their product; z2: the factors on |state|^2 from each operation on.
-void move_scalars(HostPlan* plan, const std::vector<int>& ops, const std::vector<size_t>& from, size_t keeper,
-                  std::vector<double>* z2) {
-    const cl total = product_of_scalars(plan, ops, from, keeper);
-    cl f;
+// by their product.
+void move_scalars(std::vector<ScalarOp>& ops, const std::vector<size_t>& from, size_t keeper) {
+    const Scalar total = product_of_scalars(ops, from, keeper);
     for (size_t i : from) {
-        KOp& o = plan->ops[ops[i]];
-        double* c = plan->coef.data() + o.coef;
-        if (i == keeper || !scalar_of(o, c, &f)) continue;
-        (*z2)[i] /= static_cast<double>(std::norm(f));
+        if (i == keeper) continue;
+        KOp& o = *ops[i].o;
+        double* c = ops[i].c;
+        ops[i].z2 /= ops[i].f.norm();
         if (o.kind == K_REAL) {
             c[1] /= c[0];
             c[2] /= c[0];
@@ -1336,23 +1374,29 @@ void move_scalars(HostPlan* plan, const std::vector<int>& ops, const std::vector
             c[0] = 1.0;
             o.special = SP_UNIT;
         } else {
-            const cl d1 = cl(c[2], c[3]) / f;
+            const Scalar conj{ops[i].f.re, -ops[i].f.im};
+            const Scalar d1 = Scalar{{c[2], 0.0}, {c[3], 0.0}} * conj;
+            const Dd n = ops[i].f.re * ops[i].f.re + ops[i].f.im * ops[i].f.im;
             c[0] = 1.0;
             c[1] = 0.0;
-            c[2] = static_cast<double>(d1.real());
-            c[3] = static_cast<double>(d1.imag());
+            c[2] = (d1.re / n).h;
+            c[3] = (d1.im / n).h;
             o.flags |= F_D0_ONE;
         }
     }
-    if (total == cl(1.0L, 0.0L)) return;
-    const KOp& o = plan->ops[ops[keeper]];
-    double* c = plan->coef.data() + o.coef;
+    if (total.one()) return;
+    const KOp& o = *ops[keeper].o;
+    double* c = ops[keeper].c;
     if (o.kind == K_REAL || o.kind == K_RX) {
-        for (int i = 0; i < (o.kind == K_REAL ? 4 : 2); ++i) c[i] = static_cast<double>(c[i] * total.real());
+        for (int i = 0; i < (o.kind == K_REAL ? 4 : 2); ++i) c[i] = (Dd{c[i], 0.0} * total.re).h;
     } else {
-        scale_complex(c, o.kind == K_DIAG ? 2 : free_scalar_coefs(o, false), total);
+        for (int i = 0; i < (o.kind == K_DIAG ? 2 : free_scalar_coefs(o, false)); ++i) {
+            const Scalar v = Scalar{{c[2 * i], 0.0}, {c[2 * i + 1], 0.0}} * total;
+            c[2 * i] = v.re.h;
+            c[2 * i + 1] = v.im.h;
+        }
     }
-    (*z2)[keeper] *= static_cast<double>(std::norm(total));
+    ops[keeper].z2 *= total.norm();
 }
 
 }  // namespace
@@ -1361,11 +1405,15 @@ void normalize_passes(HostPlan* plan) {
     if (!plan->binds.empty()) return;
     for (const PassDesc& pd : plan->passes) {
         if (pd.type != PASS_TILE) continue;
-        std::vector<int> ops;  // in execution order
+        std::vector<ScalarOp> ops;
         for (int si = pd.step_begin; si < pd.step_begin + pd.step_count; ++si)
-            for (int oi = 0; oi < plan->steps[si].op_count; ++oi) ops.push_back(plan->steps[si].op_begin + oi);
+            for (int oi = 0; oi < plan->steps[si].op_count; ++oi) {
+                KOp* o = &plan->ops[plan->steps[si].op_begin + oi];
+                ScalarOp s{o, plan->coef.data() + o->coef, false, {}, 1.0};
+                s.has = scalar_of(*o, s.c, &s.f);
+                ops.push_back(s);
+            }
         const NormLimits lim = pd.nprobe > 0 ? NORM_SWEEP : NORM_ONE_STATE;
-        std::vector<double> z2(ops.size(), 1.0);  // factor on |state|^2 from this op on
         // the groups, and the op of each that takes the product of the scalars
         // back: one that does so at no cost, else a phase that stays in its
         // full form, else (the product is then real) a rotation
@@ -1377,38 +1425,35 @@ void normalize_passes(HostPlan* plan) {
         bool within = true;
         for (size_t i0 = 0, i1 = 0; i0 < ops.size(); i0 = i1) {
             Group g{{}, {}, ops.size()};
-            cl f;
             for (i1 = i0; i1 < ops.size() && static_cast<int>(g.diags.size() + g.rots.size()) <= lim.count; ++i1) {
-                const KOp& o = plan->ops[ops[i1]];
-                if (free_scalar_coefs(o, pd.nprobe > 0)) g.keeper = i1;
-                if (scalar_of(o, plan->coef.data() + o.coef, &f)) (o.kind == K_DIAG ? g.diags : g.rots).push_back(i1);
+                if (free_scalar_coefs(*ops[i1].o, pd.nprobe > 0)) g.keeper = i1;
+                if (ops[i1].has) (ops[i1].o->kind == K_DIAG ? g.diags : g.rots).push_back(i1);
             }
             if (g.diags.empty() && g.rots.empty()) continue;
             if (g.keeper == ops.size()) g.keeper = !g.diags.empty() ? g.diags.back() : g.rots.back();
-            within &= in_range(product_of_scalars(plan, ops, g.rots, g.keeper) *
-                                   product_of_scalars(plan, ops, g.diags, g.keeper), lim.total);
+            within &= in_range(product_of_scalars(ops, g.rots, g.keeper) * product_of_scalars(ops, g.diags, g.keeper),
+                               lim.total);
             groups.push_back(std::move(g));
         }
         for (const Group& g : groups) {
             if (within) {
                 std::vector<size_t> all = g.diags;
                 all.insert(all.end(), g.rots.begin(), g.rots.end());
-                move_scalars(plan, ops, all, g.keeper, &z2);
+                move_scalars(ops, all, g.keeper);
                 continue;
             }
             // a phase's scalar is 1 in magnitude where the gate is unitary, a
             // rotation's NORM_MIN at least
-            if (!g.diags.empty() && in_range(product_of_scalars(plan, ops, g.diags, g.diags.back()), lim.total / NORM_MIN))
-                move_scalars(plan, ops, g.diags, g.diags.back(), &z2);
-            for (size_t k = 0; k + 1 < g.rots.size(); k += 2) move_scalars(plan, ops, {g.rots[k]}, g.rots[k + 1], &z2);
+            if (!g.diags.empty() && in_range(product_of_scalars(ops, g.diags, g.diags.back()), lim.total / NORM_MIN))
+                move_scalars(ops, g.diags, g.diags.back());
+            for (size_t k = 0; k + 1 < g.rots.size(); k += 2) move_scalars(ops, {g.rots[k]}, g.rots[k + 1]);
         }
         // reverse sweeps: both states carry the scalars taken out so far, so a
         // probe's sum carries their squared magnitude
         double z = 1.0;
         for (size_t i = 0; i < ops.size() && pd.nprobe > 0; ++i) {
-            const KOp& o = plan->ops[ops[i]];
-            if (o.kind == K_PROBE) plan->coef[o.coef] /= z;
-            z *= z2[i];
+            if (ops[i].o->kind == K_PROBE) *ops[i].c /= z;
+            z *= ops[i].z2;
         }
     }
 }
