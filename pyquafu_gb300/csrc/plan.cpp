@@ -1230,8 +1230,9 @@ namespace {
 //   one state: 2^48 leaves a factor of 2^80 to an input state far from
 //     normalised, and to Hadamards without their 1/sqrt(2);
 //   reverse sweep: a probe multiplies two states and its coefficient is
-//     divided by the square: 2^64 leaves as much to an observable, and a
-//     coefficient's low half is 2^-113 then.
+//     divided by the square: 2^72 leaves 2^56 to an observable, a coefficient's
+//     low half is 2^-121 then, and average products of 30 qubits shrunk by as
+//     much (2^-102) still have the 47 bits of a float pair.
 // A gate whose scalar is below NORM_MIN is left as it is.
 //
 // Passes that differ only in their angles have to share one compiled kernel,
@@ -1241,12 +1242,12 @@ namespace {
 // (gate by gate up to the limit, a circuit near pi met new patterns at almost
 // every step of a training).  At random angles a scalar is about 1/2 in the
 // geometric mean: 4e-8 of the gates are below NORM_MIN, 4e-6 (one state) and
-// 6e-6 (sweep) of the groups beyond their limit.
+// 4e-5 (sweep) of the groups beyond their limit.
 struct NormLimits {
     int count;
     double total;
 };
-constexpr NormLimits NORM_ONE_STATE = {15, 0x1p-48}, NORM_SWEEP = {7, 0x1p-32};
+constexpr NormLimits NORM_ONE_STATE = {15, 0x1p-48}, NORM_SWEEP = {11, 0x1p-36};
 constexpr double NORM_MIN = 0x1p-24;
 
 bool uncontrolled(const KOp& o) { return o.cthr == 0 && o.creg == 0; }

@@ -489,8 +489,8 @@ def test_sweep_probes_stay_in_single_precision(monkeypatch, precision, ansatz, n
     psi = oracle.simulate(n, ops)
     vals = helpers.interpret2(plan, psi, oracle.apply_hamiltonian(psi, terms))
     products, pair, scale = (max(w[k] for w in worst) for k in range(3))
-    # sums of products: |psi| |lam| <= 1e3 * sum |c| < 2^16, taken out: 2^-32 of each state
-    assert products < 2.0 ** 80 and scale < 2.0 ** 80
+    # sums of products: |psi| |lam| <= 1e3 * sum |c| < 2^16, taken out: 2^-36 of each state
+    assert products < 2.0 ** 88 and scale < 2.0 ** 73
     assert pair < 2.0 ** -46
     got = np.zeros(max(o.slot for o in ops) + 1)
     for v, s in zip(vals, plan["probe_slots"]):
