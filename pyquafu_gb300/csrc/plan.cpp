@@ -634,10 +634,12 @@ void keep_choices(std::string key, Choices c) {
 
 // Operations of one tile pass at most.  Fewer and larger passes are faster up
 // to where their unrolled code leaves the instruction cache, and that shows only
-// where a pass streams far more than the L2: complex64 (13, 5), depth 20 and 40,
-// 14 qubits 85 and 164 us at 45 operations, 62 and 110 without a limit; 20
-// qubits 137 and 251, 118 and 206; 25 qubits 2.05 and 3.84 ms, 1.80 and 3.49; 27
-// qubits 7.99 and 15.6 ms at 45, 7.51 and 14.2 at 62, 8.05 and 14.5 without.
+// where a pass streams far more than the L2.  Complex64 (13, 5), depth 20 and 40
+// (us): 14 qubits 85 and 164 at 45 operations, 62 and 110 at 130 or without a
+// limit; 20 qubits 137 and 251, 118 and 206; 25 qubits 2048 and 3844, 1798 and
+// 3489; 27 qubits 7988 and 15595 at 45, 7510 and 14193 at 62, 8051 and 14462 at
+// 130.  128 rather than no limit bounds the compilation, which grows faster than
+// the pass (13 qubits: 760 operations 4 s, 3800 in one pass 48 s).
 // Reverse sweeps do not depend on it (11 to 22 qubits: 2%), batched ones take
 // any number (23.3 ms at 42, 21.3 at 62, 19.1 without).  Above 26 qubits and for
 // sweeps the limits are lower than that asks for: tests/test_jit_host.py bounds
@@ -645,7 +647,8 @@ void keep_choices(std::string key, Choices c) {
 int pass_op_cap(int n, int R, bool two_states, bool bound) {
     if (bound) return INT_MAX;
     if (two_states) return R <= 3 ? 84 : 62;
-    return R >= 5 && n > 26 ? 45 : INT_MAX;
+    if (R < 5) return INT_MAX;
+    return n > 26 ? 45 : 128;
 }
 
 }  // namespace
