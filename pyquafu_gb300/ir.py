@@ -239,7 +239,7 @@ def pack(ops) -> tuple[np.ndarray, np.ndarray]:
         arr["kind"] = [o.kind for o in gates]
         arr["ncontrols"] = [o.ncontrols for o in gates]
         arr["nqubits"] = [len(o.qubits) for o in gates]
-        arr["qubits"] = [o.qubits + _QPAD[len(o.qubits)] for o in gates]
+        arr["qubits"] = [tuple(o.qubits) + _QPAD[len(o.qubits)] for o in gates]
         arr["slot"] = [o.slot for o in gates]
         arr["gen"] = [o.gen for o in gates]
         params = [tuple(o.params)[:4] for o in gates]

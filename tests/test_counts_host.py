@@ -46,3 +46,12 @@ def test_pack_records():
             assert np.array_equal(pool[r["mat_offset"]: r["mat_offset"] + m.size], m.ravel())
     with pytest.raises(ValueError):
         ir.pack([ir.Op("x", ir.OP_X, range(17))])
+
+
+@pytest.mark.parametrize("form", [list, np.array])
+def test_pack_takes_fields_set_later(form):
+    """A record's qubits and params may have been set to another sequence."""
+    op = ir.Op("rzz", ir.OP_RZZ, (0, 1), 0, (0.5,))
+    ref, _ = ir.pack([op])
+    op.qubits, op.params = form([0, 1]), form([0.5])
+    assert np.array_equal(ir.pack([op])[0], ref)
