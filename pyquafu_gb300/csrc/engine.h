@@ -268,8 +268,8 @@ bool known_unitary(const qfvm_op* ops, int64_t n_ops, const double* matpool);
 // Plans without binds: inside every tile pass, uncontrolled rotations
 // [[c, -s], [s, c]] and [[c, -is], [-is, c]] become c * (1 on the diagonal)
 // and register-bit phases d0 * diag(1, d1 / d0); the scalars' product, which
-// commutes with everything, goes back into one gate of the pass.  A rotation
-// then costs one multiply-add per real instead of a multiply and a
+// commutes with everything, goes back into one gate of a group of gates.  A
+// rotation then costs one multiply-add per real instead of a multiply and a
 // multiply-add, a phase half the amplitudes.  Probes are rescaled to match.
 void normalize_passes(HostPlan* plan);
 // The coefficient pool as complex64 kernels hold it.  Rounded coefficients
